@@ -30,7 +30,7 @@ extern std::atomic<long long> g_launches;
         CK(cudaGetLastError());                                      \
     } while (0)
 
-// Mixed-radix plan for the shared-memory Stockham FFT.
+// Radices and twiddles of the line FFT.
 struct FFTPlan {
     int n = 0;
     int nfac = 0;
@@ -110,7 +110,7 @@ struct Ctx {
     double* work = nullptr;
     FFTPlan px, py;
     // horizontal FFT: 0 = 2-D plane kernel where the grid allows it, else the
-    // tiled line kernel, else Stockham lines; 1 = tiled, else Stockham; 2 = Stockham;
+    // tiled line kernel, else the line kernel for any length; 1 = tiled, else lines; 2 = lines;
     // 3 = half-plane cluster kernel (square 64, 128), else as 0
     int fft_path = 0;
     double* gpack = nullptr;     // gathered fields, 16 doubles per grid point

@@ -19,6 +19,7 @@
 #include <vector>
 #include <algorithm>
 #include <cstring>
+#include <functional>
 #include <initializer_list>
 #include <utility>
 #include <type_traits>
@@ -28,10 +29,9 @@
 namespace epic {
 
 // ---------------------------------------------------------------------------
-// Batched real FFT of lines along x or y, one tile of T lines per CTA.
-// Two real lines are packed into one complex line (z = a + i b), transformed
-// with a mixed-radix Stockham FFT in shared memory, and separated with the
-// conjugate-symmetry identities.  Output uses the stafft Hermitian layout:
+// Real FFTs of lines along x or y.  Two real lines are packed into one complex
+// line (z = a + i b), transformed, and separated with the conjugate-symmetry
+// identities.  Output uses the stafft Hermitian layout:
 //   out[k] = Re X_k / sqrt(n) (k <= n/2),  out[n-k] = Im X_k / sqrt(n).
 constexpr int MAXF = 12;
 
@@ -41,142 +41,13 @@ struct FFTBatch {
     long long es;          // element stride along the transformed axis
     long long row_stride;  // stride between rows of lines
     int nl;                // lines per row (nz + 1, contiguous)
-    int T;                 // lines per tile (even)
+    int T;                 // lines per tile (even; a power of two for k_fft_lines)
     int n;
     int nfac;
     int fac[16];
     const double2* tw;
     double scale;
 };
-
-EPIC_DEV double2 cmul(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-EPIC_DEV double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-EPIC_DEV double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-
-// Stockham autosort passes on L complex lines of length n held in a / b.
-// Returns the buffer holding the result.
-EPIC_DEV double2* stockham(double2* a, double2* b, int L, int n, int nfac, const int* fac,
-                           const double2* tw) {
-    int Ns = 1;
-    for (int s = 0; s < nfac; ++s) {
-        int p = fac[s];
-        int m = n / p;
-        int tstep = n / (Ns * p);
-        for (int idx = threadIdx.x; idx < L * m; idx += blockDim.x) {
-            int l2 = idx / m, j = idx - l2 * m;
-            int k = j % Ns;
-            const double2* src = a + (long long)l2 * n;
-            double2* dst = b + (long long)l2 * n;
-            double2 v[5];
-            for (int r = 0; r < p; ++r) v[r] = src[j + r * m];
-            for (int r = 1; r < p; ++r) v[r] = cmul(v[r], tw[(k * r * tstep) % n]);
-            double2 o[5];
-            if (p == 2) {
-                o[0] = cadd(v[0], v[1]);
-                o[1] = csub(v[0], v[1]);
-            } else if (p == 4) {
-                double2 t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-                double2 t2 = cadd(v[1], v[3]), d = csub(v[1], v[3]);
-                double2 t3 = make_double2(d.y, -d.x);   // -i * d
-                o[0] = cadd(t0, t2);
-                o[2] = csub(t0, t2);
-                o[1] = cadd(t1, t3);
-                o[3] = csub(t1, t3);
-            } else {
-                int step = n / p;
-                for (int q = 0; q < p; ++q) {
-                    double2 acc = v[0];
-                    for (int r = 1; r < p; ++r) acc = cadd(acc, cmul(v[r], tw[((q * r) % p) * step]));
-                    o[q] = acc;
-                }
-            }
-            int base = (j / Ns) * Ns * p + k;
-            for (int r = 0; r < p; ++r) dst[base + r * Ns] = o[r];
-        }
-        __syncthreads();
-        double2* t = a; a = b; b = t;
-        Ns *= p;
-    }
-    return a;
-}
-
-template <bool FWD, class TI, class TO>
-__global__ void __launch_bounds__(256) k_fft_lines(FFTBatch B) {
-    extern __shared__ double smem[];
-    const int n = B.n, T = B.T, L = T / 2;
-    double* sx = smem;
-    double2* cz = reinterpret_cast<double2*>(sx + (long long)T * n);
-    double2* cw = cz + (long long)L * n;
-    double2* stw = cw + (long long)L * n;
-    const TI* in = static_cast<const TI*>(B.in[blockIdx.z]);
-    TO* out = static_cast<TO*>(B.out[blockIdx.z]);
-    const int l0 = blockIdx.x * T;
-    const long long rowbase = (long long)blockIdx.y * B.row_stride + 1;
-
-    for (int i = threadIdx.x; i < n; i += blockDim.x) stw[i] = B.tw[i];
-    for (int idx = threadIdx.x; idx < T * n; idx += blockDim.x) {
-        int l = idx % T, e = idx / T;
-        int line = l0 + l;
-        sx[e * T + l] = (line < B.nl) ? (double)in[rowbase + line + (long long)e * B.es] : 0.0;
-    }
-    __syncthreads();
-    const int h = n / 2;
-    if (FWD) {
-        for (int idx = threadIdx.x; idx < L * n; idx += blockDim.x) {
-            int l2 = idx / n, e = idx - l2 * n;
-            cz[idx] = make_double2(sx[e * T + 2 * l2], sx[e * T + 2 * l2 + 1]);
-        }
-    } else {
-        // Hermitian lines a, b -> conj(Xa + i Xb)
-        for (int idx = threadIdx.x; idx < L * n; idx += blockDim.x) {
-            int l2 = idx / n, k = idx - l2 * n;
-            int la = 2 * l2, lb = la + 1;
-            double ra, ia, rb, ib;
-            if (k == 0 || k == h) {
-                ra = sx[k * T + la]; ia = 0.0;
-                rb = sx[k * T + lb]; ib = 0.0;
-            } else if (k < h) {
-                ra = sx[k * T + la]; ia = sx[(n - k) * T + la];
-                rb = sx[k * T + lb]; ib = sx[(n - k) * T + lb];
-            } else {
-                ra = sx[(n - k) * T + la]; ia = -sx[k * T + la];
-                rb = sx[(n - k) * T + lb]; ib = -sx[k * T + lb];
-            }
-            cz[idx] = make_double2(ra - ib, -(ia + rb));
-        }
-    }
-    __syncthreads();
-    double2* res = stockham(cz, cw, L, n, B.nfac, B.fac, stw);
-    if (FWD) {
-        for (int idx = threadIdx.x; idx < L * (h + 1); idx += blockDim.x) {
-            int l2 = idx / (h + 1), k = idx - l2 * (h + 1);
-            double2 zk = res[(long long)l2 * n + k];
-            double2 zn = res[(long long)l2 * n + ((n - k) % n)];
-            int la = 2 * l2, lb = la + 1;
-            sx[k * T + la] = 0.5 * (zk.x + zn.x);
-            sx[k * T + lb] = 0.5 * (zk.y + zn.y);
-            if (k > 0 && k < h) {
-                sx[(n - k) * T + la] = 0.5 * (zk.y - zn.y);
-                sx[(n - k) * T + lb] = 0.5 * (zn.x - zk.x);
-            }
-        }
-    } else {
-        for (int idx = threadIdx.x; idx < L * n; idx += blockDim.x) {
-            int l2 = idx / n, e = idx - l2 * n;
-            double2 z = res[idx];
-            sx[e * T + 2 * l2] = z.x;
-            sx[e * T + 2 * l2 + 1] = -z.y;
-        }
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < T * n; idx += blockDim.x) {
-        int l = idx % T, e = idx / T;
-        int line = l0 + l;
-        if (line < B.nl) out[rowbase + line + (long long)e * B.es] = (TO)(sx[e * T + l] * B.scale);
-    }
-}
 
 // ---------------------------------------------------------------------------
 // 2-D plane FFT: one CTA transforms one (field, z) plane of an n x n grid
@@ -296,6 +167,194 @@ template <int N, class T>
 EPIC_DEV void fft_any(CX<T> (&v)[N]) {
     if constexpr ((N & (N - 1)) == 0) fft_reg<N>(v);
     else fft_reg3<N>(v);
+}
+
+// cos(2 pi j / n) to the last bit or two, for constants: the angle is reduced to
+// [0, pi / 4] in whole numbers, then the Taylor series.
+constexpr double cos_sin_series(double x, bool sine) {
+    double term = sine ? x : 1.0, sum = term;
+    for (int k = sine ? 2 : 1; k < 24; k += 2) {
+        term *= -x * x / (double)(k * (k + 1));
+        sum += term;
+    }
+    return sum;
+}
+constexpr double cos_turn(int j, int n) {
+    j %= n;
+    if (2 * j > n) j = n - j;                                          // cos is even
+    if (4 * j > n) return -cos_turn(n - 2 * j, 2 * n);                 // cos(pi - x)
+    const double x = 2.0 * 3.14159265358979323846 * (double)j / (double)n;
+    if (8 * j <= n) return cos_sin_series(x, false);
+    return cos_sin_series(2.0 * 3.14159265358979323846 * (double)(n - 4 * j) / (double)(4 * n), true);
+}
+constexpr double sin_turn(int j, int n) { return cos_turn(4 * j + 3 * n, 4 * n); }   // cos(x - pi / 2)
+template <int N>
+struct Turns {
+    double c[N], s[N];
+    constexpr Turns() : c(), s() {
+        for (int j = 0; j < N; ++j) { c[j] = cos_turn(j, N); s[j] = sin_turn(j, N); }
+    }
+};
+
+// Forward DFT of N values in registers, N = 2^a 3^b 5^c <= 16 (natural order in
+// and out): N = A B by DFTs of length A over the decimated subsequences,
+// twiddles, and DFTs of length B.
+template <int N, class T>
+EPIC_DEV void dft(CX<T> (&v)[N]) {
+    if constexpr ((N & (N - 1)) == 0) {
+        fft_reg<N>(v);
+    } else if constexpr (N == 3) {
+        const T h = (T)C30;   // sqrt(3) / 2
+        const CX<T> s = v[1] + v[2], d = v[1] - v[2];
+        const CX<T> m = cx<T>(v[0].x - T(0.5) * s.x, v[0].y - T(0.5) * s.y);
+        v[0] = v[0] + s;
+        v[1] = cx<T>(m.x + h * d.y, m.y - h * d.x);
+        v[2] = cx<T>(m.x - h * d.y, m.y + h * d.x);
+    } else if constexpr (N == 5) {
+        constexpr double c1 = cos_turn(1, 5), c2 = cos_turn(2, 5), s1 = sin_turn(1, 5), s2 = sin_turn(2, 5);
+        const CX<T> p1 = v[1] + v[4], m1 = v[1] - v[4], p2 = v[2] + v[3], m2 = v[2] - v[3], a = v[0];
+        const CX<T> r1 = cx<T>(a.x + (T)c1 * p1.x + (T)c2 * p2.x, a.y + (T)c1 * p1.y + (T)c2 * p2.y);
+        const CX<T> r2 = cx<T>(a.x + (T)c2 * p1.x + (T)c1 * p2.x, a.y + (T)c2 * p1.y + (T)c1 * p2.y);
+        const CX<T> i1 = cx<T>((T)s1 * m1.x + (T)s2 * m2.x, (T)s1 * m1.y + (T)s2 * m2.y);
+        const CX<T> i2 = cx<T>((T)s2 * m1.x - (T)s1 * m2.x, (T)s2 * m1.y - (T)s1 * m2.y);
+        v[0] = a + p1 + p2;
+        v[1] = cx<T>(r1.x + i1.y, r1.y - i1.x);   // r - i im
+        v[4] = cx<T>(r1.x - i1.y, r1.y + i1.x);
+        v[2] = cx<T>(r2.x + i2.y, r2.y - i2.x);
+        v[3] = cx<T>(r2.x - i2.y, r2.y + i2.x);
+    } else {
+        constexpr int A = N % 5 == 0 ? 5 : 3, B = N / A;
+        constexpr Turns<N> W;
+        CX<T> u[B][A];
+#pragma unroll
+        for (int b = 0; b < B; ++b) {
+#pragma unroll
+            for (int a = 0; a < A; ++a) u[b][a] = v[b + B * a];
+            dft<A>(u[b]);
+#pragma unroll
+            for (int a = 1; a < A; ++a)
+                if (b > 0) u[b][a] = cmulw(u[b][a], cx<T>((T)W.c[a * b], (T)-W.s[a * b]));
+        }
+#pragma unroll
+        for (int a = 0; a < A; ++a) {
+            CX<T> y[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b) y[b] = u[b][a];
+            dft<B>(y);
+#pragma unroll
+            for (int b = 0; b < B; ++b) v[a + A * b] = y[b];
+        }
+    }
+}
+
+// Line FFT for any even length with factors 2, 3, 5: a CTA holds T consecutive
+// z-lines of one y (x) index in shared memory, in FP64, as z[e * T/2 + p]: the
+// complex line p is the line pair (2p, 2p + 1), so the real lines are z fastest as
+// in the fields and no access transposes.  The complex lines are transformed in
+// place, decimating in frequency, in stages of radix R <= 16: a thread takes the
+// R elements of one butterfly of one line pair (the lanes of a warp run over the
+// pairs) into registers, so a length of up to 256 passes through shared memory
+// twice.  The result is in digit-reversed order, undone by the slot table when
+// it is stored.  Bound by the latency of these passes (small tiles, many CTAs).
+constexpr int LT = 128;   // threads
+template <int R>
+EPIC_DEV void line_stage(CX<double>* z, const CX<double>* tw, int n, int lnp, int len) {
+    const int np = 1 << lnp, M = len / R, ts = n / len;
+    for (int i = threadIdx.x; i < (n / R) << lnp; i += LT) {
+        const int u = i >> lnp, b = u / M, j = u - b * M;
+        CX<double>* e = z + ((b * len + j) << lnp) + (i & (np - 1));
+        CX<double> v[R];
+#pragma unroll
+        for (int m = 0; m < R; ++m) v[m] = e[(m * M) << lnp];
+        dft<R>(v);
+        if (M > 1) {
+#pragma unroll
+            for (int q = 1; q < R; ++q) v[q] = cmulw(v[q], tw[j * q * ts]);
+        }
+#pragma unroll
+        for (int q = 0; q < R; ++q) e[(q * M) << lnp] = v[q];
+    }
+}
+
+template <bool FWD, class TI, class TO>
+__global__ void __launch_bounds__(LT, 4) k_fft_lines(FFTBatch B) {
+    extern __shared__ __align__(16) double smem[];
+    const int n = B.n, T = B.T, lt = 31 - __clz(T), lnp = lt - 1, np = T >> 1, h = n / 2;
+    CX<double>* z = reinterpret_cast<CX<double>*>(smem);
+    CX<double>* tw = z + n * np;
+    unsigned short* slot = reinterpret_cast<unsigned short*>(tw + n);
+    const int l0 = blockIdx.x * T;
+    const long long row = (long long)blockIdx.y * B.row_stride + 1 + l0;
+    const TI* in = static_cast<const TI*>(B.in[blockIdx.z]) + row;
+    TO* out = static_cast<TO*>(B.out[blockIdx.z]) + row;
+    const int live = B.nl - l0;   // lines of this tile that exist
+    for (int i = threadIdx.x; i < n; i += LT) {
+        tw[i] = cx<double>(B.tw[i].x, B.tw[i].y);
+        int k = i, len = n, at = 0;
+        for (int s = 0; s < B.nfac; ++s) {
+            const int r = B.fac[s], q = k / r;
+            len /= r;
+            at += (k - q * r) * len;
+            k = q;
+        }
+        slot[i] = (unsigned short)at;
+    }
+#pragma unroll 8
+    for (int i = threadIdx.x; i < n << lt; i += LT) {
+        const int l = i & (T - 1);
+        smem[i] = l < live ? (double)in[l + (long long)(i >> lt) * B.es] : 0.0;
+    }
+    __syncthreads();
+    if (!FWD) {
+        // Hermitian lines a, b -> conj(Xa + i Xb), elements k and n - k
+        for (int i = threadIdx.x; i < (h + 1) << lnp; i += LT) {
+            const int k = i >> lnp, p = i & (np - 1);
+            CX<double>& u = z[(k << lnp) + p];
+            if (k == 0 || k == h) {
+                u.y = -u.y;
+            } else {
+                CX<double>& w = z[((n - k) << lnp) + p];
+                const CX<double> r = u, m = w;
+                u = cx<double>(r.x - m.y, -(m.x + r.y));
+                w = cx<double>(r.x + m.y, m.x - r.y);
+            }
+        }
+        __syncthreads();
+    }
+    int len = n;
+    for (int s = 0; s < B.nfac; ++s) {
+        switch (B.fac[s]) {
+            case 2: line_stage<2>(z, tw, n, lnp, len); break;
+            case 3: line_stage<3>(z, tw, n, lnp, len); break;
+            case 4: line_stage<4>(z, tw, n, lnp, len); break;
+            case 5: line_stage<5>(z, tw, n, lnp, len); break;
+            case 6: line_stage<6>(z, tw, n, lnp, len); break;
+            case 8: line_stage<8>(z, tw, n, lnp, len); break;
+            case 9: line_stage<9>(z, tw, n, lnp, len); break;
+            case 10: line_stage<10>(z, tw, n, lnp, len); break;
+            case 12: line_stage<12>(z, tw, n, lnp, len); break;
+            default: line_stage<16>(z, tw, n, lnp, len); break;
+        }
+        len /= B.fac[s];
+        __syncthreads();
+    }
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n << lt; i += LT) {
+        const int l = i & (T - 1), e = i >> lt, p = l >> 1;
+        if (l >= live) continue;
+        double v;
+        if (FWD) {
+            const int k = e <= h ? e : n - e;
+            const CX<double> zk = z[(slot[k] << lnp) + p], zn = z[(slot[k == 0 ? 0 : n - k] << lnp) + p];
+            if (e <= h) v = l & 1 ? zk.y + zn.y : zk.x + zn.x;
+            else v = l & 1 ? zn.x - zk.x : zk.y - zn.y;
+            v *= 0.5;
+        } else {
+            const CX<double> q = z[(slot[e] << lnp) + p];
+            v = l & 1 ? -q.y : q.x;
+        }
+        out[l + (long long)e * B.es] = (TO)(v * B.scale);
+    }
 }
 
 template <int N> struct Radix;
@@ -778,10 +837,30 @@ static void make_plan(FFTPlan& p, int n, cudaStream_t st) {
     p.n = n;
     p.nfac = 0;
     int rem = n;
-    for (int f : {4, 2, 3, 5})
-        while (rem % f == 0) { p.fac[p.nfac++] = f; rem /= f; }
+    for (int f : {2, 3, 5})
+        while (rem % f == 0) rem /= f;
     if (rem != 1 || n % 2 != 0)
         throw CudaError(EPIC_ERR_CONFIG, "horizontal grid sizes must be even and factor into 2, 3, 5");
+    // radices: the fewest stages, then the smallest largest radix
+    for (int stages = 1; p.nfac == 0; ++stages) {
+        int best = 17, at[16];
+        std::function<void(int, int, int)> pick = [&](int left, int k, int largest) {
+            if (k == stages) {
+                if (left == 1 && largest < best) {
+                    best = largest;
+                    p.nfac = stages;
+                    std::copy(at, at + stages, p.fac);
+                }
+                return;
+            }
+            for (int r : {16, 12, 10, 9, 8, 6, 5, 4, 3, 2})
+                if (left % r == 0 && (k == 0 || r <= at[k - 1])) {
+                    at[k] = r;
+                    pick(left / r, k + 1, std::max(largest, r));
+                }
+        };
+        pick(n, 0, 0);
+    }
     std::vector<double2> tw(n);
     for (int m = 0; m < n; ++m) {
         double a = -2.0 * M_PI * (double)m / (double)n;
@@ -791,10 +870,12 @@ static void make_plan(FFTPlan& p, int n, cudaStream_t st) {
     CK(cudaMemcpyAsync(p.tw, tw.data(), sizeof(double2) * n, cudaMemcpyHostToDevice, st));
 }
 
-static int tile_lines(int n) {
-    int T = 4096 / n;
-    T = std::max(2, std::min(32, T));
-    return T & ~1;
+// z-lines per tile of k_fft_lines: 32 or 16, which pads nl less (32 on a tie),
+// fewer where the tile would take more than 64 KB of shared memory.
+static int tile_lines(int nl, int n) {
+    int T = (nl + 31) / 32 * 32 <= (nl + 15) / 16 * 16 ? 32 : 16;
+    while (T > 2 && sizeof(double) * (size_t)T * n > 64 * 1024) T /= 2;
+    return T;
 }
 
 template <class TI, class TO>
@@ -808,22 +889,21 @@ static void run_fft_axis(Ctx& c, const FFTPlan& pl, int axis, const TI* const* i
     for (int k = 0; k < 16; ++k) B.fac[k] = pl.fac[k];
     B.tw = pl.tw;
     B.nl = P.nz + 1;
-    B.T = tile_lines(pl.n);
+    B.T = tile_lines(B.nl, pl.n);
     B.scale = 1.0 / std::sqrt((double)pl.n);
     int nrows;
     if (axis == 0) { B.es = (long long)P.ny * P.nzh; B.row_stride = P.nzh; nrows = P.ny; }
     else { B.es = P.nzh; B.row_stride = (long long)P.ny * P.nzh; nrows = P.nx; }
-    size_t sm = sizeof(double) * (size_t)B.T * B.n + 2 * sizeof(double2) * (size_t)(B.T / 2) * B.n +
-                sizeof(double2) * B.n;
+    size_t sm = sizeof(double) * (size_t)B.T * B.n + (sizeof(double2) + sizeof(unsigned short)) * (size_t)B.n;
     dim3 grid((B.nl + B.T - 1) / B.T, nrows, nf);
     prof_begin(c, "fft");
     if (forward) {
         allow_smem(k_fft_lines<true, TI, TO>, sm);
-        k_fft_lines<true, TI, TO><<<grid, 256, sm, c.stream>>>(B);
+        k_fft_lines<true, TI, TO><<<grid, LT, sm, c.stream>>>(B);
         CKL();
     } else {
         allow_smem(k_fft_lines<false, TI, TO>, sm);
-        k_fft_lines<false, TI, TO><<<grid, 256, sm, c.stream>>>(B);
+        k_fft_lines<false, TI, TO><<<grid, LT, sm, c.stream>>>(B);
         CKL();
     }
     prof_end(c, "fft");
@@ -838,7 +918,7 @@ void fft_xy(Ctx& c, const TI* const* in, TO* const* out, int nf, bool forward) {
         int k = std::min(MAXF, nf - f0);
         if (c.fft_path == 3 && half_fft(c, in + f0, out + f0, k, forward)) continue;
         if ((c.fft_path == 0 || c.fft_path == 3) && plane_fft(c, in + f0, out + f0, k, forward)) continue;
-        // per axis: tiled register FFT for powers of two up to 256, else Stockham lines
+        // per axis: tiled register FFT where it has the length, else the line FFT
         auto axis = [&](const FFTPlan& pl, int ax, auto src, TO* const* dst, bool fwd) {
             if (c.fft_path <= 1 && tile_axis(c, pl, ax, src, dst, k, fwd)) return;
             run_fft_axis(c, pl, ax, src, dst, k, fwd);

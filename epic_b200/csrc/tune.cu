@@ -53,7 +53,7 @@ void autotune(Ctx& c, epic_tuning* out) {
     }
     c.scatter_lg[1] = c.scatter_lg[2] = best_p;
     c.scatter_lg[0] = best_v;
-    // horizontal FFT path: plane kernel (square grids up to 128), tiled lines, Stockham lines,
+    // horizontal FFT path: plane kernel (square grids up to 128), tiled lines, lines of any length,
     // half-plane cluster kernel (square 64 and 128)
     int best_f = c.fft_path;
     float tf = FLT_MAX;

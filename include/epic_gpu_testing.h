@@ -42,7 +42,7 @@ int epic_gpu_test_reflective_bc(struct epic_ctx* ctx);
 /* Selects the horizontal FFT implementation of the context: 0 (default) the
  * 2-D plane kernel for square grids of 16, 32, 64 or 128 points, else the
  * tiled line kernel; 1 the tiled line kernel (power-of-two axes 16 .. 256);
- * 2 the batched Stockham line kernels (any even size with factors 2, 3, 5);
+ * 2 the batched line kernels (any even size with factors 2, 3, 5);
  * 3 the half-plane kernel (a cluster of two CTAs per plane, square 64 or 128).
  * Each falls back to the next where it does not apply; all compute
  * fftxyp2s / fftxys2p (sta3dfft.f90:134-257). */
