@@ -6,19 +6,20 @@
 // parcel of every box is recorded.  One CTA takes one box; parcels appended
 // later (split children) are handled in tail chunks of SCHUNK parcels.
 //
-// Scatter (parcel_interpl.f90:160-233): every contribution w * v of a support
-// point (trilinear weight w of a corner, value v = attribute x point weight
-// 1/4 x volume) is a fixed-point integer q = round(w v s_f) at one scale
-// s_f = 2^(b - e_f) per field and launch, 2^e_f above the largest |v| of the
-// field over all parcels (a bound computed before the scatter).  Grid sums
-// are integer sums, exact and therefore independent of the order of the adds:
-// par2grid is bitwise reproducible run to run and for any launch shape.  A box
-// CTA adds its parcels' contributions into a shared-memory window (the box's
-// grid points and WM more on every side) as three 32-bit limbs with integer
-// shared atomics, then adds the window to the 64-bit integer grid sums held in
-// the field arrays; points outside the window, and tail chunks whose parcels
-// do not fit a window, add to the grid sums directly.  The tail kernels
-// (parcels.cu) fold the z halos in integers and convert to FP64.
+// Scatter (parcel_interpl.f90:160-233): the runs of a warp's 32 consecutive
+// parcels (a run is the support points of one parcel in one cell, its trilinear
+// weights summed) are grouped by cell and every group's 8 corners x fields are
+// summed as an FP64 matrix product, in the order of the parcels.  Each group
+// sum is then a fixed-point integer q = round(d s_f) at one scale
+// s_f = 2^(b - e_f) per field and launch, 2^e_f above the largest |value| of
+// the field over all parcels (a bound computed before the scatter).  Grid sums
+// are 64-bit integer sums, exact and therefore independent of the order in
+// which warps add: par2grid is bitwise reproducible run to run for a given
+// parcel order.  A box CTA adds into a shared-memory window (the box's grid
+// points and WM more on every side), then adds the window to the 64-bit
+// integer grid sums held in the field arrays; points outside the window, and
+// tail chunks whose parcels do not fit a window, add to the grid sums directly.
+// The tail kernels (parcels.cu) fold the z halos in integers and convert to FP64.
 //
 // Stage (ls_rk.f90:142-217 + parcel_interpl.f90:405-470): grid2par at the
 // support points (support vectors stored by the preceding scatter, from the
@@ -35,18 +36,18 @@ namespace epic {
 constexpr int BOXX = 8, BOXY = 4, BOXZ = 4;   // cells per box
 constexpr int BOXC = BOXX * BOXY * BOXZ;
 constexpr int SCHUNK = 2048;    // parcels per tail chunk
-constexpr int ROUND = 4096;     // parcels per fixed-point round
 // Window of a box CTA: the box's grid points and WM more on every side
-// (parcels that moved up to a cell out of the box since the sort, plus half
-// a cell of support-point reach), 13 x 9 x 9 grid points.
-constexpr int WM = 2;
-constexpr int WCAP = (BOXX + 1 + 2 * WM) * (BOXY + 1 + 2 * WM) * (BOXZ + 1 + 2 * WM);
-// Words per limb plane: at least WCAP, and 11 banks apart (WSTRIDE = 11 mod
-// 32), so that two lanes adding different limbs of the same grid point hit
-// different banks (see LimbOrder).
-constexpr int WSTRIDE = ((WCAP + 31 - 11) / 32) * 32 + 11;
-constexpr int NLIMB = 3;
-constexpr int SB = 2;           // CTAs per SM the scatter kernels are sized for
+// (support points up to a cell outside the box), 11 x 7 x 7 grid points.  The
+// extents are compile-time constants: the flush walks the window without
+// divisions by run-time numbers.
+constexpr int WM = 1;
+constexpr int WX = BOXX + 1 + 2 * WM, WY = BOXY + 1 + 2 * WM, WZ = BOXZ + 1 + 2 * WM;
+constexpr int WCAP = WX * WY * WZ;
+// Words per plane (a window sum is two words in two planes): at least WCAP, and
+// 17 banks apart, so that a field's two planes are 2 banks from the next
+// field's and the 8 corners x 4 fields of one flush instruction meet in few banks.
+constexpr int WSTRIDE = ((WCAP + 31 - 17) / 32) * 32 + 17;
+constexpr int SB = 2;           // CTAs per SM the stage kernel is sized for
 
 // Box ranges of the sorted parcel store.
 struct Boxes {
@@ -58,7 +59,6 @@ struct Boxes {
 
 struct Window {
     int gx0, gy0, gz0;   // window origin (grid point; x, y unwrapped)
-    int WX, WY, WZ;      // extents
     int ok;
 };
 
@@ -117,17 +117,14 @@ struct WinShared {
     double scale[NF];
 };
 
-// Window of a box CTA: fixed, the box's grid points +- WM (z clipped to the
-// halo rows -1 .. nz + 1).
+// Window of a box CTA: the box's grid points +- WM (rows outside the halo rows
+// -1 .. nz + 1 stay empty).
 EPIC_DEV Window box_window(const Params& P, const Range& R) {
     Window W;
     W.gx0 = R.ref[0] - WM;
     W.gy0 = R.ref[1] - WM;
-    W.gz0 = max(R.ref[2] - WM, -1);
-    W.WX = BOXX + 1 + 2 * WM;
-    W.WY = BOXY + 1 + 2 * WM;
-    W.WZ = min(R.ref[2] + BOXZ + WM, P.nz + 1) - W.gz0 + 1;
-    W.ok = W.WX <= P.nx && W.WY <= P.ny;   // no grid point twice in one window
+    W.gz0 = R.ref[2] - WM;
+    W.ok = WX <= P.nx && WY <= P.ny;   // no grid point twice in one window
     return W;
 }
 
@@ -160,23 +157,18 @@ EPIC_DEV Window tail_window(const Params& P, const Range& R, const int* mn, cons
     Window W;
     W.gx0 = R.ref[0] + mn[0] - 1;
     W.gy0 = R.ref[1] + mn[1] - 1;
-    W.gz0 = max(R.ref[2] + mn[2] - 1, -1);
-    W.WX = mx[0] - mn[0] + 4;
-    W.WY = mx[1] - mn[1] + 4;
-    W.WZ = min(R.ref[2] + mx[2] + 2, P.nz + 1) - W.gz0 + 1;
-    W.ok = mn[0] <= mx[0] && W.WX <= P.nx && W.WY <= P.ny && W.WZ > 0 && (long long)W.WX * W.WY * W.WZ <= WCAP;
+    W.gz0 = R.ref[2] + mn[2] - 1;
+    W.ok = mn[0] <= mx[0] && WX <= P.nx && WY <= P.ny && mx[0] - mn[0] + 4 <= WX && mx[1] - mn[1] + 4 <= WY &&
+           mx[2] - mn[2] + 4 <= WZ;
     return W;
 }
 
 struct Fields7 {
     double* f[7];   // vortg x,y,z, dbuoyg, humg, tbuoyg, volg (64-bit integer sums during the scatter)
-    int mask;       // bit f set: field f is accumulated (NF = 7)
 };
-constexpr int ALL_FIELDS = 0x7f;
-constexpr int DRY_FIELDS = 0x67;   // without dbuoyg (3) and humg (4)
 
-// Field set of a scatter kernel: NF = 7 (all, masked by Fields7.mask), 5 (the
-// dry set: vorticity, tbuoyg, volg) or 1 (one field, vol2grid).
+// Field set of a scatter kernel: NF = 7 (all), 5 (the dry set: vorticity,
+// tbuoyg, volg) or 1 (one field, vol2grid).
 template <int NF>
 EPIC_HD constexpr int field_slot(int f) {
     return NF == 5 ? (f < 3 ? f : f + 2) : f;
@@ -187,11 +179,6 @@ template <int NF>
 EPIC_HD constexpr int bound_slot(int f) {
     return NF == 1 ? 6 : field_slot<NF>(f);
 }
-template <int NF>
-EPIC_DEV bool field_on(const Fields7& F, int f) {
-    return NF != 7 || ((F.mask >> f) & 1);
-}
-
 // Arithmetic of the two forms: R is the type of the FP32-able attributes,
 // of the gathered values and of the window sums (double: plain, float: mixed).
 template <class R> struct Form {
@@ -215,17 +202,19 @@ EPIC_DEV R& aR(const PView& pv, int k, long long i) {
                                 (Form<R>::mixed ? mixed_slot_off(k) : 8LL * k) * pv.cap)[i];
 }
 
-// Fixed-point bits: |w v s_f| <= 2^(b + 2) (merged weights of up to 4 support
-// points).  Plain: b = 46, three window limbs (18 + 18 bits unsigned and a
-// signed top), 4 x ROUND contributions per grid point per round within 32
-// bits each, 2^15 contributions per grid point within the 64-bit grid sums;
-// rounding 2^-47 of the field's largest value.  Mixed: b = 34, two limbs
-// (19 bits unsigned and a signed top) for 4 x 2048 contributions per round,
-// far below FP32 rounding.
+// Fixed-point bits: |w v s_f| <= 2^(b + 2) for a run (merged weights of up to 4
+// support points), 2^(b + 7) for a group; 2^15 full parcels per grid point fit
+// the 64-bit grid sums.  Plain: b = 46, each sum rounded by at most 2^-47 of the
+// field's largest value.  Mixed: b = 34, far below FP32 rounding.
+//
+// Window sums are two 32-bit words (the hardware has no native 64-bit shared
+// add).  Plain: the halves of a 64-bit sum; the low word is added first and its
+// carry goes with the high word (three 18-bit limbs without a carry: 15% more
+// time).  Mixed: 19 low bits and a signed top, no carry, for 4 x 2048 adds per
+// grid point between two flushes.
 template <class R> constexpr int fx_bits() { return Form<R>::mixed ? 34 : 46; }
-template <class R> constexpr int win_words() { return Form<R>::mixed ? 2 : NLIMB; }
-template <class R, int NF> constexpr size_t win_bytes() { return sizeof(unsigned) * NF * win_words<R>() * WSTRIDE; }
-template <class R> constexpr int round_max() { return Form<R>::mixed ? 2048 : ROUND; }
+template <int NF> constexpr size_t win_bytes() { return sizeof(unsigned) * NF * 2 * WSTRIDE; }
+template <class R> constexpr int round_max() { return Form<R>::mixed ? 2048 : INT_MAX; }
 
 // Scale of field slot k from its bound (largest |value| as ordered bits).
 EPIC_DEV double fx_scale(const unsigned long long* pbound, int k, int bits, unsigned* err) {
@@ -239,81 +228,170 @@ EPIC_DEV double fx_scale(const unsigned long long* pbound, int k, int bits, unsi
     return ldexp(1.0, bits - e);
 }
 
-// Rounding of w * vs (|w vs| <= 2^50) to an integer: r = w vs + 1.5 * 2^52
-// rounds once; the low 52 bits of r hold 2^51 + q.
-constexpr double FX_MAGIC = 6755399441055744.0;   // 1.5 * 2^52
-EPIC_DEV long long fx_round(double wt, double vs) {
-    const double r = fma(wt, vs, FX_MAGIC);
-    return (__double_as_longlong(r) & 0xfffffffffffffll) - (1ll << 51);
-}
-
-// The order in which a lane adds the limbs of a contribution.  The two lanes
-// of a lane pair take consecutive parcels, usually of one cell, so at every
-// corner they add to the same grid point: the odd lane adds its limbs in
-// rotated order, and with the limb planes 11 banks apart the pair's atomics
-// of one instruction hit different banks instead of the same word.  The
-// sums do not depend on the order.
-struct LimbOrder {
-    int p0, p1, p2;   // plane offsets (words) of the 1st, 2nd and 3rd add
-    bool rot;
-    EPIC_DEV explicit LimbOrder(int nlimb) {
-        rot = (threadIdx.x & 1) != 0;
-        if (nlimb == 3) {
-            p0 = rot ? WSTRIDE : 0;
-            p1 = rot ? 2 * WSTRIDE : WSTRIDE;
-            p2 = rot ? 0 : 2 * WSTRIDE;
-        } else {
-            p0 = rot ? WSTRIDE : 0;
-            p1 = rot ? 0 : WSTRIDE;
-            p2 = 0;
-        }
+// A sum d, rounded to an integer q, into the window; and the window's sum.
+template <class R>
+EPIC_DEV void fx_add(unsigned* acc, double d) {
+    const unsigned long long q = (unsigned long long)__double2ll_rn(d);
+    if constexpr (Form<R>::mixed) {
+        atomicAdd(&acc[0], (unsigned)q & 0x7ffffu);
+        atomicAdd(&acc[WSTRIDE], (unsigned)(q >> 19));
+    } else {
+        const unsigned lo = (unsigned)q, old = atomicAdd(&acc[0], lo);
+        atomicAdd(&acc[WSTRIDE], (unsigned)(q >> 32) + (unsigned)(old > ~lo));
     }
-};
-
-// q = ((m >> 36) - 2^15) * 2^36 + ((m >> 18) & 0x3ffff) * 2^18 + (m & 0x3ffff), m = 2^51 + q
-EPIC_DEV void fx_add(unsigned* acc, int w, double wt, double vs, const LimbOrder& o) {
-    double r = fma(wt, vs, FX_MAGIC);
-    unsigned lo = (unsigned)__double2loint(r), hi = (unsigned)__double2hiint(r);
-    const unsigned l0 = lo & 0x3ffffu;
-    const unsigned l1 = (lo >> 18) | ((hi & 0xfu) << 14);
-    const unsigned l2 = ((hi & 0xfffffu) >> 4) - 32768u;
-    atomicAdd(&acc[o.p0 + w], o.rot ? l1 : l0);
-    atomicAdd(&acc[o.p1 + w], o.rot ? l2 : l1);
-    atomicAdd(&acc[o.p2 + w], o.rot ? l0 : l2);
 }
-EPIC_DEV long long fx_sum(const unsigned* acc, int w) {
-    return (long long)(int)acc[2 * WSTRIDE + w] * (1ll << 36) + (long long)acc[WSTRIDE + w] * (1ll << 18) +
-           (long long)acc[w];
+// A product w v of one run, |w v| <= 2^48: the sum w v + 1.5 * 2^52 is rounded at
+// the units place and its bits are those of the constant plus q (no conversion
+// instruction, which runs at an eighth of the rate).
+template <class R>
+EPIC_DEV void fx_add_product(unsigned* acc, double w, double v) {
+    const double r = fma(w, v, 6755399441055744.0);
+    const unsigned lo = (unsigned)__double2loint(r), hi = (unsigned)__double2hiint(r) - 0x43380000u;
+    if constexpr (Form<R>::mixed) {
+        atomicAdd(&acc[0], lo & 0x7ffffu);
+        atomicAdd(&acc[WSTRIDE], __funnelshift_r(lo, hi, 19));
+    } else {
+        const unsigned old = atomicAdd(&acc[0], lo);
+        atomicAdd(&acc[WSTRIDE], hi + (unsigned)(old > ~lo));
+    }
 }
-
-// Two-limb variant: q = h * 2^19 + l, l = q mod 2^19, h = floor(q / 2^19).
-EPIC_DEV void fx2_add(unsigned* acc, int w, double wt, double vs, const LimbOrder& o) {
-    double r = fma(wt, vs, FX_MAGIC);
-    long long m = __double_as_longlong(r) & 0xfffffffffffffll;   // 2^51 + q
-    const unsigned l0 = (unsigned)(m & 0x7ffff);
-    const unsigned l1 = (unsigned)((m >> 19) - (1ll << 32));
-    atomicAdd(&acc[o.p0 + w], o.rot ? l1 : l0);
-    atomicAdd(&acc[o.p1 + w], o.rot ? l0 : l1);
-}
-EPIC_DEV long long fx2_sum(const unsigned* acc, int w) {
-    return (long long)(int)acc[WSTRIDE + w] * (1ll << 19) + (long long)acc[w];
+template <class R>
+EPIC_DEV long long fx_sum(const unsigned* acc) {
+    if constexpr (Form<R>::mixed) return (long long)(int)acc[WSTRIDE] * (1ll << 19) + (long long)acc[0];
+    else return (long long)((unsigned long long)acc[WSTRIDE] << 32 | acc[0]);
 }
 
-// A contribution straight into the 64-bit grid sum of field f at point g.
-EPIC_DEV void fx_global(double* f, long long g, double wt, double vs) {
-    const long long q = fx_round(wt, vs);
+// A group sum straight into the 64-bit grid sum of field f at point g.
+EPIC_DEV void fx_global(double* f, long long g, double d) {
+    const long long q = __double2ll_rn(d);
     if (q != 0) atomicAdd(reinterpret_cast<unsigned long long*>(f) + g, (unsigned long long)q);
 }
 
-EPIC_DEV int wrap_to(int l, int n) { return ((unsigned)l < (unsigned)n) ? l : wrapi(l, n); }
+// l modulo n; support points rarely lie more than a period off the grid
+EPIC_DEV int wrap_to(int l, int n) {
+    l += l < 0 ? n : 0;
+    l -= l >= n ? n : 0;
+    return (unsigned)l < (unsigned)n ? l : wrapi(l, n);
+}
 
-// Support points of one parcel that fall into the same cell as the point
-// before them share their 8 corners: their trilinear weights are summed and
-// the corners visited once (sum_p w_p f = (sum_p w_p) f; only the rounding
-// order differs from visiting each point).
-EPIC_DEV bool same_cell(const Tri& a, const Tri& b) { return a.is == b.is && a.js == b.js && a.ks == b.ks; }
+// Floor of x as a double rounded down at the units place: the low word of
+// x + 1.5 * 2^52 is the floor as an int, and subtracting the constant again
+// gives it as a double (two additions instead of a rounding and two
+// conversions, which run at an eighth of the FP64 rate).
+constexpr double FLOOR_MAGIC = 6755399441055744.0;   // 1.5 * 2^52
+EPIC_DEV double floor_bits(double x) { return __dadd_rd(x, FLOOR_MAGIC); }
+EPIC_DEV int floor_int(double t) { return __double2loint(t); }
+
+// The 4 support points of a parcel in cells from the domain's corner
+// (parcel_ellipsoid.f90:216-260, interpl.f90:17-56): centre u, points u + a,
+// u - b, u - a, u + b with a = (eta + tau) / sqrt 2, b = (eta - tau) / sqrt 2.
+struct Points {
+    double u[3], a[3], b[3];
+    EPIC_DEV void set(const Params& P, const double* pos, const double* eta, const double* tau) {
+        const double r = 0.70710678118654752440;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            u[k] = (pos[k] - P.lower[k]) * P.dxi[k];
+            const double s = r * P.dxi[k];
+            a[k] = s * (eta[k] + tau[k]);
+            b[k] = s * (eta[k] - tau[k]);
+        }
+    }
+    // Whether the points lie where floor_bits' low word is their cell (a NaN or
+    // infinite position does not).
+    EPIC_DEV bool z_near() const { return fabs(u[2]) + fabs(a[2]) + fabs(b[2]) < 1.0e9; }
+    template <int Q>
+    EPIC_DEV double at(int k) const {
+        return Q == 0 ? u[k] + a[k] : Q == 1 ? u[k] - b[k] : Q == 2 ? u[k] - a[k] : u[k] + b[k];
+    }
+};
+
+// The 4 points grouped by cell: bits 4 q .. 4 q + 3 hold the points in the cell
+// of point q, q included, that follow no earlier point of that cell.
+EPIC_DEV int point_groups(const Points& p) {
+    int d01 = 0, d02 = 0, d03 = 0, d12 = 0, d13 = 0, d23 = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int c0 = floor_int(floor_bits(p.at<0>(k))), c1 = floor_int(floor_bits(p.at<1>(k)));
+        const int c2 = floor_int(floor_bits(p.at<2>(k))), c3 = floor_int(floor_bits(p.at<3>(k)));
+        d01 |= c0 ^ c1; d02 |= c0 ^ c2; d03 |= c0 ^ c3;
+        d12 |= c1 ^ c2; d13 |= c1 ^ c3; d23 |= c2 ^ c3;
+    }
+    return 0x8421 | (d01 ? 0 : 0x2) | (d02 ? 0 : 0x4) | (d03 ? 0 : 0x8) | (d12 ? 0 : 0x40) | (d13 ? 0 : 0x80) |
+           (d23 ? 0 : 0x800);
+}
+
+// A run: the points of a parcel in one cell, as the sums over them of the
+// products of their offsets x, y, z from the cell's corner, in which the
+// trilinear weights of the corners are linear (sum_p w_p f = (sum_p w_p) f).
+struct Run {
+    int c[3];
+    double n, x, y, z, xy, xz, yz, xyz;
+    EPIC_DEV void add(const Points& p, int q) {
+        double f[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double o = q & 1 ? p.b[k] : p.a[k];
+            const double X = q == 1 || q == 2 ? p.u[k] - o : p.u[k] + o, t = floor_bits(X);
+            c[k] = floor_int(t);
+            f[k] = X - (t - FLOOR_MAGIC);
+        }
+        const double fxy = f[0] * f[1];
+        n += 1.0;
+        x += f[0]; y += f[1]; z += f[2];
+        xy += fxy;
+        xz = fma(f[0], f[2], xz);
+        yz = fma(f[1], f[2], yz);
+        xyz = fma(fxy, f[2], xyz);
+    }
+    // All 4 points: as they come in pairs u +- a, u +- b, the sums are a few
+    // products of u's offset, a and b, a quarter of the arithmetic of 4 points.
+    EPIC_DEV void all(const Points& p) {
+        double f[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const double t = floor_bits(p.at<0>(k));
+            c[k] = floor_int(t);
+            f[k] = p.u[k] - (t - FLOOR_MAGIC);
+        }
+        const double pxy = 2.0 * fma(p.a[0], p.a[1], p.b[0] * p.b[1]);
+        const double pxz = 2.0 * fma(p.a[0], p.a[2], p.b[0] * p.b[2]);
+        const double pyz = 2.0 * fma(p.a[1], p.a[2], p.b[1] * p.b[2]);
+        n = 4.0;
+        x = 4.0 * f[0]; y = 4.0 * f[1]; z = 4.0 * f[2];
+        xy = fma(x, f[1], pxy);
+        xz = fma(x, f[2], pxz);
+        yz = fma(y, f[2], pyz);
+        xyz = fma(xy, f[2], fma(f[0], pyz, f[1] * pxz));
+    }
+    // The points of mask m (in one cell).
+    EPIC_DEV void set(const Points& p, int m) {
+        if (m == 15) return all(p);
+        n = x = y = z = xy = xz = yz = xyz = 0.0;
+        for (; m; m &= m - 1) add(p, __ffs(m) - 1);
+    }
+    // Measure the offsets from the other end of the axes in flip (bits 4, 2, 1:
+    // x, y, z): the corner weights w[k] are then those of the corners k ^ flip.
+    EPIC_DEV void flip(int m) {
+        if (m & 4) { x = n - x; xy = y - xy; xz = z - xz; xyz = yz - xyz; }
+        if (m & 2) { y = n - y; xy = x - xy; yz = z - yz; xyz = xz - xyz; }
+        if (m & 1) { z = n - z; xz = x - xz; yz = y - yz; xyz = xy - xyz; }
+    }
+    // w[4 i + 2 j + k]: corner (i, j, k) in x, y, z
+    EPIC_DEV void weights(double* w) const {
+        w[7] = xyz;
+        w[6] = xy - xyz;
+        w[5] = xz - xyz;
+        w[3] = yz - xyz;
+        w[4] = (x - xy) - w[5];
+        w[2] = (y - xy) - w[3];
+        w[1] = (z - xz) - w[3];
+        w[0] = (((n - x) - y) + xy) - w[1];
+    }
+};
+
 // Whether point p lies in t's cell, and if so adds its trilinear weights to
-// t's (the arithmetic of trilinear() followed by add_weights(), without a
+// t's (the arithmetic of trilinear() followed by adding its weights, without a
 // second Tri held in registers).
 EPIC_DEV bool merge_into(const Params& P, const double* p, Tri& t) {
     const double x = (p[0] - P.lower[0]) * P.dxi[0];
@@ -328,14 +406,6 @@ EPIC_DEV bool merge_into(const Params& P, const double* p, Tri& t) {
     t.w[0][0][0] += pzc * w00; t.w[0][0][1] += pzc * w10; t.w[0][1][0] += pzc * w01; t.w[0][1][1] += pzc * w11;
     t.w[1][0][0] += pz * w00;  t.w[1][0][1] += pz * w10;  t.w[1][1][0] += pz * w01;  t.w[1][1][1] += pz * w11;
     return true;
-}
-EPIC_DEV void add_weights(Tri& a, const Tri& b) {
-#pragma unroll
-    for (int kk = 0; kk < 2; ++kk)
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-            for (int ii = 0; ii < 2; ++ii) a.w[kk][jj][ii] += b.w[kk][jj][ii];
 }
 EPIC_DEV void support_point(const double* pos, const double* eta, const double* tau, int p, double* pt) {
     const double cp = support_cos(p), sp = support_sin(p);
@@ -362,79 +432,170 @@ EPIC_DEV int merge_start(const Params& P, const double* pos, const double* eta, 
     return 0;
 }
 
-// Scatter one support point (or the merged points of one parcel in one cell):
-// vs[f] = value x volume x point weight x s_f.
+// D += A B on the FP64 tensor path: A 8 x 4 (lane: row lane / 4, column
+// lane % 4), B 4 x 8 (row lane % 4, column lane / 4), D 8 x 8 (row lane / 4,
+// columns 2 (lane % 4) and the next).
+EPIC_DEV void mma_f64(double& d0, double& d1, double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(d0), "+d"(d1) : "d"(a), "d"(b));
+}
+
+// The most cells among a warp's runs, and the fewest runs per cell, for which
+// the matrix products of scatter_groups are used: below three runs per cell the
+// groups' sums cost more than adding every product.
+constexpr int MAX_GROUPS = 8, MIN_MATES = 3;
+// Staging rows of one warp: the corner weights (8) of one run per lane, the values (NF) of its parcel, and the groups.
+// The row strides (10, and 6 or 10 doubles) make the 16-byte stores of a quarter
+// warp conflict-free.  Row 32 stays zero: it pads the groups to whole row quads.
+template <int NF>
+struct alignas(16) WarpRows {
+    static constexpr int WS = 10, VS = NF <= 5 ? 6 : 10;
+    double w[33 * WS];
+    double v[33 * VS];
+    int2 group[MAX_GROUPS];     // cell code; first member | row quads << 8
+    unsigned char member[64];   // lanes in group order
+    EPIC_DEV void clear_pad(int lane) {
+        if (lane < WS) w[32 * WS + lane] = 0.0;
+        if (lane < VS) v[32 * VS + lane] = 0.0;
+    }
+};
+template <> struct WarpRows<1> {
+    EPIC_DEV void clear_pad(int) {}
+};
+template <int NF> constexpr size_t rows_bytes() { return NF == 1 ? 0 : sizeof(WarpRows<NF>) * (PB / 32); }
+
+// Grid point of a corner of a cell outside the window; code is the complement
+// of the periodic cell number.
+struct FarCell {
+    int x, y, z;
+    EPIC_DEV FarCell(const Params& P, int code) {
+        const int id = ~code, xy = id / P.nzh;
+        z = id - xy * P.nzh;
+        x = xy / P.ny;
+        y = xy - x * P.ny;
+    }
+    EPIC_DEV long long point(const Params& P, int corner) const {
+        const int X = x + (corner >> 2), Y = y + ((corner >> 1) & 1);
+        return ((long long)(X == P.nx ? 0 : X) * P.ny + (Y == P.ny ? 0 : Y)) * P.nzh + z + (corner & 1);
+    }
+};
+// A cell as a code: >= 0, the window point of its corner 0, or < 0, the
+// complement of its periodic cell number.
+EPIC_DEV int cell_code(const Params& P, const Window& W, const int* c) {
+    const int lx = wrap_to(c[0] - W.gx0, P.nx), ly = wrap_to(c[1] - W.gy0, P.ny), lz = c[2] - W.gz0;
+    if (W.ok && lx + 1 < WX && ly + 1 < WY && lz >= 0 && lz + 1 < WZ) return (lx * WY + ly) * WZ + lz;
+    return ~((wrap_to(c[0], P.nx) * P.ny + wrap_to(c[1], P.ny)) * P.nzh + c[2] + 1);
+}
+EPIC_DEV int corner_offset(int corner) { return ((corner >> 2) * WY + ((corner >> 1) & 1)) * WZ + (corner & 1); }
+
+// The runs of a warp's lanes as matrix products, one run (cell code, corner
+// weights w) per active lane: the runs are grouped by cell and each group's 8
+// corners x NF fields are weights (8 x 4) times values (4 x NF) summed over its
+// runs, four per instruction; only the sums are rounded and added with atomics
+// (adding each product takes 16 NF atomics per run).  mates: the lanes of the
+// same cell; leads: the first lane of each cell.
 template <int NF, class R>
-EPIC_DEV void scatter_tri(const Params& P, const Window& W, unsigned* acc, const Fields7& F, const Tri& t,
-                          const double* vs, const LimbOrder& lo, unsigned* err) {
-    if (t.ks < -1 || t.ks > P.nz) { set_err(err, ERRB_ZRANGE); return; }
-    int lx = wrap_to(t.is - W.gx0, P.nx), ly = wrap_to(t.js - W.gy0, P.ny), lz = t.ks - W.gz0;
-    if (W.ok && lx + 1 < W.WX && ly + 1 < W.WY && lz >= 0 && lz + 1 < W.WZ) {
-        int base = (lx * W.WY + ly) * W.WZ + lz;
+EPIC_DEV void scatter_groups(const Params& P, unsigned* acc, const Fields7& F, bool active, int code, unsigned mates,
+                             unsigned leads, const double* w, WarpRows<NF>* rows) {
+    using WR = WarpRows<NF>;
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const bool lead = active && (mates & below) == 0;
+    // The lanes in group order, padded with row 32: the first member of each
+    // group is the exclusive sum of the padded sizes over the leads.
+    const int quads = (__popc(mates) + 3) >> 2;
+    int sum = lead ? quads : 0;
 #pragma unroll
-        for (int ii = 0; ii < 2; ++ii)
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += u;
+    }
+    const int first = 4 * __shfl_sync(0xffffffffu, sum - (lead ? quads : 0), active ? __ffs(mates) - 1 : 0);
+    __syncwarp();   // the rows of the previous call are read
+    reinterpret_cast<unsigned short*>(rows->member)[lane] = 0x2020;
+    __syncwarp();
+    if (active) {
+        rows->member[first + __popc(mates & below)] = (unsigned char)lane;
+        double2* wr = reinterpret_cast<double2*>(rows->w + lane * WR::WS);
 #pragma unroll
-            for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-                    int w = base + (ii * W.WY + jj) * W.WZ + kk;
-                    if constexpr (Form<R>::mixed) {
-                        const double wt = (double)(float)t.w[kk][jj][ii];
-#pragma unroll
-                        for (int f = 0; f < NF; ++f)
-                            if (field_on<NF>(F, f)) fx2_add(acc + f * 2 * WSTRIDE, w, wt, vs[f], lo);
-                    } else {
-                        const double wt = t.w[kk][jj][ii];
-#pragma unroll
-                        for (int f = 0; f < NF; ++f)
-                            if (field_on<NF>(F, f)) fx_add(acc + f * NLIMB * WSTRIDE, w, wt, vs[f], lo);
-                    }
-                }
-    } else {
-        long long a[2][2];
-        corners(P, t, a);
-#pragma unroll
-        for (int ii = 0; ii < 2; ++ii)
-#pragma unroll
-            for (int jj = 0; jj < 2; ++jj)
-#pragma unroll
-                for (int kk = 0; kk < 2; ++kk) {
-                    long long g = a[jj][ii] + kk;
-                    const double wt = Form<R>::mixed ? (double)(float)t.w[kk][jj][ii] : t.w[kk][jj][ii];
-#pragma unroll
-                    for (int f = 0; f < NF; ++f)
-                        if (field_on<NF>(F, f)) fx_global(F.f[field_slot<NF>(f)], g, wt, vs[f]);
-                }
+        for (int k = 0; k < 4; ++k) wr[k] = make_double2(w[2 * k], w[2 * k + 1]);
+    }
+    if (lead) rows->group[__popc(leads & below)] = make_int2(code, first | (quads << 8));
+    __syncwarp();
+    const int ng = __popc(leads);
+    const int r4 = lane >> 2, c4 = lane & 3, f = 2 * c4;
+    // columns past the fields repeat the last one and are dropped
+    const double *wl = rows->w + r4, *vl = rows->v + min(r4, NF - 1);
+    unsigned* al = acc + f * 2 * WSTRIDE + corner_offset(r4);
+    for (int g = 0; g < ng; ++g) {
+        const int2 gr = rows->group[g];
+        const unsigned char* ml = rows->member + (gr.y & 0xff) + c4;
+        double d0 = 0.0, d1 = 0.0;
+        for (int k = gr.y >> 8; k > 0; --k, ml += 4) {
+            const int m = *ml;
+            mma_f64(d0, d1, wl[m * WR::WS], vl[m * WR::VS]);
+        }
+        if (gr.x >= 0) {
+            if (f < NF) fx_add<R>(al + gr.x, d0);
+            if (f + 1 < NF) fx_add<R>(al + gr.x + 2 * WSTRIDE, d1);
+        } else {
+            const long long g = FarCell(P, gr.x).point(P, r4);
+            if (f < NF) fx_global(F.f[field_slot<NF>(f)], g, d0);
+            if (f + 1 < NF) fx_global(F.f[field_slot<NF>(f + 1)], g, d1);
+        }
     }
 }
 
+// Every product of a run on its own: weights of the corners c ^ flip.  Lanes of
+// one cell have different flips, so that one instruction adds to different
+// grid points of the cell instead of serialising on one.
 template <int NF, class R>
-EPIC_DEV void win_zero(unsigned* acc, const Window& W) {
-    if (!W.ok) return;
-    int n = W.WX * W.WY * W.WZ;
-    for (int f = 0; f < NF * win_words<R>(); ++f)
-        for (int w = threadIdx.x; w < n; w += blockDim.x) acc[f * WSTRIDE + w] = 0u;
+EPIC_DEV void scatter_products(const Params& P, unsigned* acc, const Fields7& F, int code, int flip, const double* w,
+                               const double* v) {
+    if (code >= 0) {
+        // offsets of the axes' far corners, from the flipped corner 0
+        const int sx = flip & 4 ? -WY * WZ : WY * WZ, sy = flip & 2 ? -WZ : WZ, sz = flip & 1 ? -1 : 1;
+        unsigned* a0 = acc + code + corner_offset(flip);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            unsigned* a = a0 + (k & 4 ? sx : 0) + (k & 2 ? sy : 0) + (k & 1 ? sz : 0);
+#pragma unroll
+            for (int f = 0; f < NF; ++f) fx_add_product<R>(a + f * 2 * WSTRIDE, w[k], v[f]);
+        }
+    } else {
+        const FarCell far(P, code);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const long long g = far.point(P, k ^ flip);
+#pragma unroll
+            for (int f = 0; f < NF; ++f) fx_global(F.f[field_slot<NF>(f)], g, w[k] * v[f]);
+        }
+    }
 }
 
-// The window's integer sums into the 64-bit grid sums.
+template <int NF>
+EPIC_DEV void win_zero(unsigned* acc, const Window& W) {
+    if (!W.ok) return;
+    uint4* a = reinterpret_cast<uint4*>(acc);
+    for (int w = threadIdx.x; w < (int)((win_bytes<NF>() + 15) / 16); w += blockDim.x) a[w] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+// The window's integer sums into the 64-bit grid sums.  Window points lie less
+// than one period outside the grid (W.ok: the window is not wider than it).
 template <int NF, class R>
 EPIC_DEV void win_flush(const Params& P, const unsigned* acc, const Window& W, const Fields7& F) {
     if (!W.ok) return;
-    int n = W.WX * W.WY * W.WZ;
-    for (int w = threadIdx.x; w < n; w += blockDim.x) {
-        int z = w % W.WZ;
-        int r = w / W.WZ;
-        int y = r % W.WY;
-        int x = r / W.WY;
-        long long g = fidx(P, W.gz0 + z, wrapi(W.gy0 + y, P.ny), wrapi(W.gx0 + x, P.nx));
+    for (int w = threadIdx.x; w < WCAP; w += blockDim.x) {
+        const int z = w % WZ, r = w / WZ;
+        int y = W.gy0 + r % WY, x = W.gx0 + r / WY;
+        y += y < 0 ? P.ny : y >= P.ny ? -P.ny : 0;
+        x += x < 0 ? P.nx : x >= P.nx ? -P.nx : 0;
+        const long long g = fidx(P, W.gz0 + z, y, x);
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-            if (!field_on<NF>(F, f)) continue;
-            long long q;
-            if constexpr (Form<R>::mixed) q = fx2_sum(acc + f * 2 * WSTRIDE, w);
-            else q = fx_sum(acc + f * NLIMB * WSTRIDE, w);
-            if (q != 0) atomicAdd(reinterpret_cast<unsigned long long*>(F.f[field_slot<NF>(f)]) + g,
-                                  (unsigned long long)q);
+            const long long q = fx_sum<R>(acc + f * 2 * WSTRIDE + w);
+            if (q != 0)
+                atomicAdd(reinterpret_cast<unsigned long long*>(F.f[field_slot<NF>(f)]) + g, (unsigned long long)q);
         }
     }
 }
@@ -443,8 +604,9 @@ EPIC_DEV void win_flush(const Params& P, const unsigned* acc, const Window& W, c
 // value * point weight (1/4) * volume.
 template <class R>
 EPIC_DEV void p2g_values(const Params& P, const R* vor, double z, double vol, R buoy, R hum, R* vp) {
-    R q_c = hum - (R)P.q_0 * exp((R)(P.lambda_c * (P.lower[2] - z)));
-    q_c = fmax((R)0, q_c);
+    // max(0, h - saturation): dry parcels (h <= 0) skip the exponential
+    R q_c = (R)0;
+    if (hum > (R)0) q_c = fmax((R)0, hum - (R)P.q_0 * exp((R)(P.lambda_c * (P.lower[2] - z))));
     const R pw = (R)(0.25 * vol);
     vp[0] = pw * vor[0];
     vp[1] = pw * vor[1];
@@ -539,42 +701,123 @@ EPIC_DEV void vectors(const PView& pv, long long i, bool reuse, bool store, R* e
     }
 }
 
-// The support points of parcels [q0, q1) into the window (or the grid sums).
+// The support points of parcels [q0, q1) into the window (or the grid sums):
+// a warp takes 32 consecutive parcels, one per lane.
 template <int NF, class R, bool VEC = true>
-EPIC_DEV void scatter_round(const Params& P, const PView& pv, long long q0, long long q1, const WinShared<NF>* ws,
-                            unsigned* acc, const Fields7& F, int* nparg, int* nsparg, bool reuse, bool store,
-                            int lg, unsigned* err) {
+EPIC_DEV void scatter_parcels(const Params& P, const PView& pv, long long q0, long long q1, const WinShared<NF>* ws,
+                              unsigned* acc, WarpRows<NF>* rows, const Fields7& F, int* nparg, int* nsparg, bool reuse,
+                              bool store, unsigned* err) {
     const Window W = ws->W;
-    // The lanes of a warp take groups of 2^lg consecutive parcels spaced about
-    // cnt/32 * 2^lg apart (different cells of the box), so that the addresses
-    // of one shared-memory atomic spread over the banks (consecutive parcels
-    // of one cell would pile onto few), while a group still shares sectors
-    // of the parcel loads.
-    const int cnt = (int)(q1 - q0);
-    const int U = (cnt + (1 << lg) - 1) >> lg;          // groups
-    const int cols = 32 >> lg;                          // groups side by side in a warp
-    const int S = (U + cols - 1) / cols;                // groups per column
-    const int lane = threadIdx.x & 31, gi = lane >> lg, m = lane & ((1 << lg) - 1);
-    const LimbOrder lo(win_words<R>());
-    for (int r = threadIdx.x >> 5; r < S; r += blockDim.x >> 5) {
-        const int u = gi * S + r;
-        const int slot = (u << lg) + m;
-        if (u >= U || slot >= cnt) continue;
-        long long i = q0 + slot;
-        double pos[3] = {a64<R>(pv, A_X, i), a64<R>(pv, A_Y, i), a64<R>(pv, A_Z, i)};
-        R eta[3], tau[3];
-        // VEC: the support vectors may be recomputed here; else they are stored
-        vectors<R>(pv, i, VEC ? reuse : true, store, eta, tau, err);
-        double vs[NF];
-        {
+    const int lane = threadIdx.x & 31;
+    for (long long ib = q0 + (threadIdx.x & ~31); ib < q1; ib += blockDim.x) {
+        const long long i = ib + lane;
+        Points pts;
+        double v[NF];
+        int todo = 0, same = 0;   // support points left; the points of each cell
+        if constexpr (NF != 1) __syncwarp();   // the values of the previous parcels are read
+        if (i < q1) {
+            const double pos[3] = {a64<R>(pv, A_X, i), a64<R>(pv, A_Y, i), a64<R>(pv, A_Z, i)};
+            R eta[3], tau[3];
+            // VEC: the support vectors may be recomputed here; else they are stored
+            vectors<R>(pv, i, VEC ? reuse : true, store, eta, tau, err);
             R vp[NF];
             load_values<NF, R>(P, pv, i, pos[2], vp);
 #pragma unroll
-            for (int f = 0; f < NF; ++f) vs[f] = (double)vp[f] * ws->scale[f];
+            for (int l = 0; l < NF; ++l) v[l] = (double)vp[l] * ws->scale[l];
+            if constexpr (NF != 1) {
+                double* vr = rows->v + lane * WarpRows<NF>::VS;
+#pragma unroll
+                for (int l = 0; l + 1 < NF; l += 2) *reinterpret_cast<double2*>(vr + l) = make_double2(v[l], v[l + 1]);
+                vr[NF - 1] = v[NF - 1];
+                if (nparg) count_parcel(P, pos, a64<R>(pv, A_VOL, i), nparg, nsparg, err);
+            }
+            const double ed[3] = {(double)eta[0], (double)eta[1], (double)eta[2]};
+            const double td[3] = {(double)tau[0], (double)tau[1], (double)tau[2]};
+            pts.set(P, pos, ed, td);
+            same = point_groups(pts);
+            if (pts.z_near()) todo = 15;
+            else set_err(err, ERRB_ZRANGE);
         }
-        if (NF != 1 && nparg) count_parcel(P, pos, a64<R>(pv, A_VOL, i), nparg, nsparg, err);
+        while (__any_sync(0xffffffffu, todo != 0)) {
+            bool active = todo != 0;
+            Run run;
+            int code = 0;
+            if (active) {
+                const int m = same >> (4 * (__ffs(todo) - 1)) & 15;
+                todo &= ~m;
+                run.set(pts, m);
+                if (run.c[2] < -1 || run.c[2] > P.nz) { set_err(err, ERRB_ZRANGE); active = false; }
+                else code = cell_code(P, W, run.c);
+            }
+            bool groups = false;
+            unsigned mates = 0, leads = 0;
+            if constexpr (NF != 1) {
+                const unsigned act = __ballot_sync(0xffffffffu, active);
+                if (active) mates = __match_any_sync(act, code);
+                leads = __ballot_sync(0xffffffffu, active && (mates & ((1u << lane) - 1u)) == 0);
+                groups = __popc(leads) <= MAX_GROUPS && MIN_MATES * __popc(leads) <= __popc(act);
+            }
+            const int flip = groups ? 0 : lane & 7;
+            double w[8];
+            if (active) {
+                run.flip(flip);
+                run.weights(w);
+            }
+            if (groups) {
+                if constexpr (NF != 1) scatter_groups<NF, R>(P, acc, F, active, code, mates, leads, w, rows);
+            } else if (active) {
+                if constexpr (NF != 1) {
+                    const double* vr = rows->v + lane * WarpRows<NF>::VS;
+#pragma unroll
+                    for (int l = 0; l < NF; ++l) v[l] = vr[l];
+                }
+                scatter_products<NF, R>(P, acc, F, code, flip, w, v);
+            }
+        }
+    }
+}
+
+// vol2grid: one value per parcel, so nothing is shared between a run's fields
+// and the lanes add their products directly, without the flips: groups of 8
+// consecutive parcels (they share load sectors) are spread over the box
+// instead, so that one instruction's atomics fall into different cells.
+template <class R, bool VEC>
+EPIC_DEV void scatter_volumes(const Params& P, const PView& pv, long long q0, long long q1, const WinShared<1>* ws,
+                              unsigned* acc, const Fields7& F, bool reuse, bool store, unsigned* err) {
+    const Window W = ws->W;
+    const int cnt = (int)(q1 - q0), U = (cnt + 7) >> 3, S = (U + 3) >> 2;   // groups, groups per 8 lanes
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < S; r += blockDim.x >> 5) {
+        const int u = (lane >> 3) * S + r, slot = (u << 3) + (lane & 7);
+        if (u >= U || slot >= cnt) continue;
+        const long long i = q0 + slot;
+        const double pos[3] = {a64<R>(pv, A_X, i), a64<R>(pv, A_Y, i), a64<R>(pv, A_Z, i)};
+        R eta[3], tau[3], vp[1];
+        vectors<R>(pv, i, VEC ? reuse : true, store, eta, tau, err);
+        load_values<1, R>(P, pv, i, pos[2], vp);
+        const double v[1] = {(double)vp[0] * ws->scale[0]};
         const double ed[3] = {(double)eta[0], (double)eta[1], (double)eta[2]};
         const double td[3] = {(double)tau[0], (double)tau[1], (double)tau[2]};
+        auto put = [&](const int* c, const double* w) {
+            if (c[2] < -1 || c[2] > P.nz) set_err(err, ERRB_ZRANGE);
+            else scatter_products<1, R>(P, acc, F, cell_code(P, W, c), 0, w, v);
+        };
+        Points pts;
+        pts.set(P, pos, ed, td);
+        if (pts.z_near() && (point_groups(pts) & 15) == 15) {
+            Run run;
+            double w[8];
+            run.all(pts);
+            run.weights(w);
+            put(run.c, w);
+            continue;
+        }
+        auto put_tri = [&](const Tri& t) {
+            const int c[3] = {t.is, t.js, t.ks};
+            const double w[8] = {t.w[0][0][0], t.w[1][0][0], t.w[0][1][0], t.w[1][1][0],
+                                 t.w[0][0][1], t.w[1][0][1], t.w[0][1][1], t.w[1][1][1]};
+            put(c, w);
+        };
         double pt[3];
         const int s0 = merge_start(P, pos, ed, td);
         support_point(pos, ed, td, s0, pt);
@@ -582,11 +825,11 @@ EPIC_DEV void scatter_round(const Params& P, const PView& pv, long long q0, long
         for (int q = 1; q < 4; ++q) {
             support_point(pos, ed, td, (s0 + q) & 3, pt);
             if (!merge_into(P, pt, cur)) {
-                scatter_tri<NF, R>(P, W, acc, F, cur, vs, lo, err);
+                put_tri(cur);
                 cur = trilinear(P, pt);
             }
         }
-        scatter_tri<NF, R>(P, W, acc, F, cur, vs, lo, err);
+        put_tri(cur);
     }
 }
 
@@ -603,19 +846,27 @@ __global__ void __launch_bounds__(PB, 4) k_vectors(PView pv, long long n, unsign
 }
 
 // par2grid scatter (NF = 7 or 5) and vol2grid (NF = 1).
+template <int NF>
+constexpr size_t scatter_bytes() {
+    return ((win_bytes<NF>() + 15) & ~(size_t)15) + rows_bytes<NF>();
+}
+// Two CTAs per SM for 5 and 7 fields: with three (80 registers, spills) the
+// 128^3 thermal gains 3% and the deformed 64^3 flow and small grids lose 4% to 9%.
 template <int NF, class R, bool VEC>
-// vol2grid (NF = 1) has a small window and few live values: three CTAs per SM
-__global__ void __launch_bounds__(PB, NF == 1 ? 3 : SB) k_scatter(Params P, PView pv, long long n, Boxes B, Fields7 F,
-                                                    const unsigned long long* pbound, int* nparg, int* nsparg,
-                                                    int reuse, int store, int lg, unsigned* err) {
+__global__ void __launch_bounds__(PB, NF == 1 ? 3 : 2) k_scatter(Params P, PView pv, long long n, Boxes B,
+                                                                 const __grid_constant__ Fields7 F,
+                                                                 const unsigned long long* pbound, int* nparg,
+                                                                 int* nsparg, int reuse, int store, unsigned* err) {
     extern __shared__ __align__(16) unsigned acc[];
     __shared__ WinShared<NF> ws;
+    constexpr size_t wbytes = (win_bytes<NF>() + 15) & ~(size_t)15;
+    WarpRows<NF>* rows = reinterpret_cast<WarpRows<NF>*>(reinterpret_cast<char*>(acc) + wbytes) + (threadIdx.x >> 5);
     const Range Rg = cta_range(P, pv, B, n);
     if (threadIdx.x == 0) {
         for (int k = 0; k < 3; ++k) { ws.mn[k] = INT_MAX; ws.mx[k] = INT_MIN; }
-        for (int f = 0; f < NF; ++f) ws.scale[f] = fx_scale(pbound, bound_slot<NF>(f), fx_bits<R>(), err);
         if (Rg.box) ws.W = box_window(P, Rg);
     }
+    if (threadIdx.x < NF) ws.scale[threadIdx.x] = fx_scale(pbound, bound_slot<NF>(threadIdx.x), fx_bits<R>(), err);
     __syncthreads();
     if (!Rg.box) {
         tail_bounds<NF>(P, Rg, pv, &ws);
@@ -623,11 +874,13 @@ __global__ void __launch_bounds__(PB, NF == 1 ? 3 : SB) k_scatter(Params P, PVie
         if (threadIdx.x == 0) ws.W = tail_window(P, Rg, ws.mn, ws.mx);
         __syncthreads();
     }
+    rows->clear_pad(threadIdx.x & 31);
     for (long long q0 = Rg.r0; q0 < Rg.r1; q0 += round_max<R>()) {
         const long long q1 = min(q0 + round_max<R>(), Rg.r1);
-        win_zero<NF, R>(acc, ws.W);
+        win_zero<NF>(acc, ws.W);
         __syncthreads();
-        scatter_round<NF, R, VEC>(P, pv, q0, q1, &ws, acc, F, nparg, nsparg, reuse != 0, store != 0, lg, err);
+        if constexpr (NF == 1) scatter_volumes<R, VEC>(P, pv, q0, q1, &ws, acc, F, reuse != 0, store != 0, err);
+        else scatter_parcels<NF, R, VEC>(P, pv, q0, q1, &ws, acc, rows, F, nparg, nsparg, reuse != 0, store != 0, err);
         __syncthreads();
         win_flush<NF, R>(P, acc, ws.W, F);
         __syncthreads();
@@ -637,8 +890,7 @@ __global__ void __launch_bounds__(PB, NF == 1 ? 3 : SB) k_scatter(Params P, PVie
 // ---------------------------------------------------------------------------
 // Fused stage kernel.
 struct FusedArgs {
-    int stage, last, lg;
-    int recwin;   // gathers from the box's records staged in shared memory (split form)
+    int stage, last;
     double ca, cb;
     // surface fluxes of stage 1 (null: none)
     const double* binc;
@@ -672,22 +924,24 @@ __global__ void k_pack_gather(GatherFields G, R* pack, long long fsz) {
     }
 }
 
-// Corner x/y indices wrapped into the grid; support points lie within a
-// cell or two of the domain, so the modulo is rarely needed.
-EPIC_DEV int wrap_near(int i, int n) {
-    if (i < 0) i += n;
-    else if (i >= n) i -= n;
-    return ((unsigned)i < (unsigned)n) ? i : wrapi(i, n);
-}
-
+// grid2par of the warp's parcels (parcel_interpl.f90:405-470): g[l] = the sum
+// over a parcel's runs and their 8 corners of w / 4 times field l (the point
+// weight 1/4), from the records of 16 values per grid point.
+//
+// One parcel per lane: every lane reads the records of its own cells.  A load
+// instruction of the warp takes a pass through L1 for each cell among the lanes,
+// few where neighbours in the store share cells.  Support points in the cell of
+// the point before them share its 8 corners: their weights are summed and the
+// corners read once.
+//
 // g[l] += sum over the 8 corners of (w / 4) f_l (interpl.f90:17-56, the
 // point weight 1/4 of parcel_interpl.f90:433).  Returns false when the
 // point leaves the vertical halo.
 template <class R>
 EPIC_DEV bool gather_tri(const Params& P, const R* __restrict__ pack, const Tri& t, R* g) {
     if (t.ks < -1 || t.ks > P.nz) return false;
-    const int i0 = wrap_near(t.is, P.nx), i1 = wrap_near(t.is + 1, P.nx);
-    const int j0 = wrap_near(t.js, P.ny), j1 = wrap_near(t.js + 1, P.ny);
+    const int i0 = wrap_to(t.is, P.nx), i1 = wrap_to(t.is + 1, P.nx);
+    const int j0 = wrap_to(t.js, P.ny), j1 = wrap_to(t.js + 1, P.ny);
 #pragma unroll
     for (int ii = 0; ii < 2; ++ii)
 #pragma unroll
@@ -720,85 +974,21 @@ EPIC_DEV bool gather_tri(const Params& P, const R* __restrict__ pack, const Tri&
     return true;
 }
 
-// Gather records of the grid points around a box, staged in shared memory by
-// the stage kernel: the cells of the box and one cell on every side, so the
-// corners of every support point within a cell of the box are on chip.
-// Records are stored whole (16 values); the 16-byte words of record r are
-// permuted by r (word w at w ^ (r mod 8), plain; w ^ (r mod 4), mixed) so
-// that the lanes of a warp, each reading word w of its own record, spread
-// over all banks.
-constexpr int RWM = 0;   // cells of margin around the box
-constexpr int RWX = BOXX + 1 + 2 * RWM, RWY = BOXY + 1 + 2 * RWM, RWZ = BOXZ + 1 + 2 * RWM;
-template <class R> constexpr int rec_words() { return (int)(GREC * sizeof(R) / 16); }   // 8 plain, 4 mixed
-template <class R> constexpr size_t recwin_bytes() { return sizeof(R) * GREC * RWX * RWY * RWZ; }
-
-struct RecWin {
-    int gx0, gy0, gz0, WZ;
-    int ok;
-};
-
 template <class R>
-EPIC_DEV RecWin recwin_load(const Params& P, const Range& Rg, bool box, const R* __restrict__ pack, R* srec) {
-    constexpr int V = rec_words<R>();
-    RecWin W;
-    W.gx0 = Rg.ref[0] - RWM;
-    W.gy0 = Rg.ref[1] - RWM;
-    W.gz0 = Rg.ref[2] - RWM;
-    W.WZ = min(RWZ, P.nz + 2 - W.gz0);
-    W.ok = box && RWX <= P.nx && RWY <= P.ny;
-    if (!W.ok) return W;
-    const int nrec = RWX * RWY * W.WZ;
-    const uint4* src = reinterpret_cast<const uint4*>(pack);
-    uint4* dst = reinterpret_cast<uint4*>(srec);
-    for (int e = threadIdx.x; e < nrec * V; e += blockDim.x) {
-        const int r = e / V, w = e - r * V;
-        const int z = r % W.WZ, xy = r / W.WZ, y = xy % RWY, x = xy / RWY;
-        const long long g = fidx(P, W.gz0 + z, wrap_near(W.gy0 + y, P.ny), wrap_near(W.gx0 + x, P.nx));
-        dst[r * V + (w ^ (r & (V - 1)))] = __ldg(src + g * V + w);
-    }
-    return W;
-}
-
-// gather_tri from the staged records when the point's corners are in the
-// window, else from global memory; the same sums in the same order.
-template <class R>
-EPIC_DEV bool gather_tri_win(const Params& P, const R* __restrict__ pack, const R* srec, const RecWin& W,
-                             const Tri& t, R* g) {
-    constexpr int V = rec_words<R>();
-    const int lx = wrap_to(t.is - W.gx0, P.nx), ly = wrap_to(t.js - W.gy0, P.ny), lz = t.ks - W.gz0;
-    if (!(W.ok && lx + 1 < RWX && ly + 1 < RWY && lz >= 0 && lz + 1 < W.WZ && t.ks >= -1 && t.ks <= P.nz))
-        return gather_tri<R>(P, pack, t, g);
-#pragma unroll
-    for (int ii = 0; ii < 2; ++ii)
-#pragma unroll
-        for (int jj = 0; jj < 2; ++jj) {
-            const int rb = ((lx + ii) * RWY + ly + jj) * W.WZ + lz;
-#pragma unroll
-            for (int kk = 0; kk < 2; ++kk) {
-                const int r = rb + kk;
-                const R w = (R)(0.25 * t.w[kk][jj][ii]);
-                if constexpr (Form<R>::mixed) {
-                    const float4* q = reinterpret_cast<const float4*>(srec) + r * V;
-#pragma unroll
-                    for (int l4 = 0; l4 < 4; ++l4) {
-                        const float4 v = q[l4 ^ (r & 3)];
-                        g[4 * l4] = fmaf(w, v.x, g[4 * l4]);
-                        g[4 * l4 + 1] = fmaf(w, v.y, g[4 * l4 + 1]);
-                        if (4 * l4 + 2 < 14) g[4 * l4 + 2] = fmaf(w, v.z, g[4 * l4 + 2]);
-                        if (4 * l4 + 3 < 14) g[4 * l4 + 3] = fmaf(w, v.w, g[4 * l4 + 3]);
-                    }
-                } else {
-                    const double2* q = reinterpret_cast<const double2*>(srec) + r * V;
-#pragma unroll
-                    for (int l2 = 0; l2 < 7; ++l2) {
-                        const double2 v = q[l2 ^ (r & 7)];
-                        g[2 * l2] = fma(w, v.x, g[2 * l2]);
-                        g[2 * l2 + 1] = fma(w, v.y, g[2 * l2 + 1]);
-                    }
-                }
-            }
+EPIC_DEV bool gather_own(const Params& P, const R* __restrict__ pack, const double* pos, const double* eta,
+                         const double* tau, int s0, R* g) {
+    double pt[3];
+    support_point(pos, eta, tau, s0, pt);
+    Tri cur = trilinear(P, pt);
+    bool ok = true;
+    for (int q = 1; q < 4; ++q) {
+        support_point(pos, eta, tau, (s0 + q) & 3, pt);
+        if (!merge_into(P, pt, cur)) {
+            ok = gather_tri<R>(P, pack, cur, g) && ok;
+            cur = trilinear(P, pt);
         }
-    return true;
+    }
+    return gather_tri<R>(P, pack, cur, g) && ok;
 }
 
 // get_dBdt (parcel_ellipsoid.f90:466-507) in the attribute type.
@@ -813,12 +1003,11 @@ EPIC_DEV void dBdt_r(const R* s, const R* b, R B33, R* o) {
 }
 
 
-template <bool DIAG, class R, bool VOUT = false>
+template <bool DIAG, class R, bool VOUT>
 __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long n, Boxes B, const R* pack,
                                                   FusedArgs S, const StepScalars* sc, double* partials,
                                                   unsigned* err) {
     using Ops = typename Form<R>::Ops;
-    extern __shared__ __align__(16) unsigned acc[];
     __shared__ double red[PB / 32][NDIAG];
     constexpr int ND = DIAG ? NDIAG : 1;
     // the diagnostic sums of this thread, in shared memory (registers are
@@ -835,13 +1024,6 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
 #define DACC(k) dacc[(k) * PB]
     const double dt = sc->dt;
     const Range Rg = cta_range(P, pv, B, n);
-    // without the scatter pass, the dynamic shared memory holds the box's gather records
-    RecWin RW;
-    RW.ok = 0;
-    if (S.recwin) {
-        RW = recwin_load<R>(P, Rg, blockIdx.x < B.nbox, pack, reinterpret_cast<R*>(acc));
-        __syncthreads();
-    }
     {
         const long long q0 = Rg.r0, q1 = Rg.r1;
         // grid2par + dB/dt + LS-RK update
@@ -862,11 +1044,16 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
             double pos[3] = {a64<R>(pv, A_X, i), a64<R>(pv, A_Y, i), a64<R>(pv, A_Z, i)};
             // the attributes of the update are loaded before the gathers, so
             // that their latency overlaps the interpolation
-            R b[5];
+            R b[5], vor[3];
+            double vol;
+            auto load_state = [&]() {
 #pragma unroll
-            for (int k = 0; k < 5; ++k) b[k] = aR<R>(pv, A_B11 + k, i);
-            const double vol = a64<R>(pv, A_VOL, i);
-            R vor[3] = {aR<R>(pv, A_VX, i), aR<R>(pv, A_VY, i), aR<R>(pv, A_VZ, i)};
+                for (int k = 0; k < 5; ++k) b[k] = aR<R>(pv, A_B11 + k, i);
+                vol = a64<R>(pv, A_VOL, i);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) vor[k] = aR<R>(pv, A_VX + k, i);
+            };
+            load_state();
             // the LS-RK accumulators: the mixed form loads them before the
             // gathers (their latency overlaps the interpolation); the FP64
             // form after them (fewer live registers, no spills)
@@ -890,20 +1077,7 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
                 for (int k = 0; k < 3; ++k) { eta[k] = aR<R>(pv, A_ETA0 + k, i); tau[k] = aR<R>(pv, A_TAU0 + k, i); }
                 const double ed[3] = {(double)eta[0], (double)eta[1], (double)eta[2]};
                 const double td[3] = {(double)tau[0], (double)tau[1], (double)tau[2]};
-                double pt[3];
-                const int s0 = merge_start(P, pos, ed, td);
-                support_point(pos, ed, td, s0, pt);
-                Tri cur = trilinear(P, pt);
-                bool ok = true;
-                for (int q = 1; q < 4; ++q) {
-                    support_point(pos, ed, td, (s0 + q) & 3, pt);
-                    if (!merge_into(P, pt, cur)) {
-                        ok = gather_tri_win<R>(P, pack, reinterpret_cast<const R*>(acc), RW, cur, g) && ok;
-                        cur = trilinear(P, pt);
-                    }
-                }
-                ok = gather_tri_win<R>(P, pack, reinterpret_cast<const R*>(acc), RW, cur, g) && ok;
-                if (!ok) set_err(err, ERRB_ZRANGE);
+                if (!gather_own<R>(P, pack, pos, ed, td, merge_start(P, pos, ed, td), g)) set_err(err, ERRB_ZRANGE);
             }
             if constexpr (!Form<R>::mixed) load_accumulators();
             double dp[3];
@@ -1040,11 +1214,10 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
 }
 
 // ---------------------------------------------------------------------------
-static Fields7 fields7(Ctx& c, bool moist = true) {
+static Fields7 fields7(Ctx& c) {
     Fields7 F;
     F.f[0] = c.vortg(0); F.f[1] = c.vortg(1); F.f[2] = c.vortg(2);
     F.f[3] = c.dbuoyg(); F.f[4] = c.humg(); F.f[5] = c.tbuoyg(); F.f[6] = c.volg();
-    F.mask = moist ? ALL_FIELDS : DRY_FIELDS;
     return F;
 }
 
@@ -1089,7 +1262,7 @@ static void set_smem(K kernel, size_t bytes) {
 
 // count: par2grid's parcel counts nparg / nsparg (NF = 7 or 5)
 template <int NF, class R>
-static void launch_scatter(Ctx& c, const Fields7& F, bool reuse, bool store, int lg, bool count) {
+static void launch_scatter(Ctx& c, const Fields7& F, bool reuse, bool store, bool count) {
     // the fixed-point scales: the largest value of every scattered field,
     // from the kernels that produced the values or from a pass of their own
     if (NF == 1 && c.v2g_bound_ready) {
@@ -1105,14 +1278,14 @@ static void launch_scatter(Ctx& c, const Fields7& F, bool reuse, bool store, int
         CKL();
         reuse = true;
     }
-    size_t sm = win_bytes<R, NF>();
+    size_t sm = scatter_bytes<NF>();
     Boxes B = boxes(c);
     int* np = count ? c.nparg : nullptr;
     int* nsp = count ? c.nsparg : nullptr;
     auto run = [&](auto kernel) {
         set_smem(kernel, sm);
-        kernel<<<sgrid(c, B), PB, sm, c.stream>>>(c.P, c.pv, c.n, B, F, c.dsc->pbound, np, nsp, reuse, store, lg,
-                                                   &c.dsc->err);
+        kernel<<<sgrid(c, B), PB, sm, c.stream>>>(c.P, c.pv, c.n, B, F, c.dsc->pbound, np, nsp, reuse, store,
+                                                  &c.dsc->err);
         CKL();
     };
     if (reuse) run(k_scatter<NF, R, false>);
@@ -1123,8 +1296,8 @@ static void launch_scatter(Ctx& c, const Fields7& F, bool reuse, bool store, int
 template <class R>
 static void launch_p2g(Ctx& c, bool moist, bool reuse, bool store, bool count) {
     c.p2g_counted = count;
-    if (moist) launch_scatter<7, R>(c, fields7(c, true), reuse, store, c.scatter_lg[1], count);
-    else launch_scatter<5, R>(c, fields7(c, false), reuse, store, c.scatter_lg[1], count);
+    if (moist) launch_scatter<7, R>(c, fields7(c), reuse, store, count);
+    else launch_scatter<5, R>(c, fields7(c), reuse, store, count);
 }
 
 void scatter_p2g(Ctx& c, bool reuse, bool store, bool moist) {
@@ -1141,10 +1314,9 @@ void scatter_v2g(Ctx& c, bool reuse) {
     if (c.n == 0) return;
     Fields7 F;
     F.f[0] = c.volg();
-    F.mask = 1;
     prof_begin(c, "v2g");
-    if (c.pv.mixed) launch_scatter<1, float>(c, F, reuse, true, c.scatter_lg[0], false);
-    else launch_scatter<1, double>(c, F, reuse, true, c.scatter_lg[0], false);
+    if (c.pv.mixed) launch_scatter<1, float>(c, F, reuse, true, false);
+    else launch_scatter<1, double>(c, F, reuse, true, false);
     prof_end(c, "v2g");
 }
 
@@ -1179,7 +1351,6 @@ static void launch_stage(Ctx& c, const FusedArgs& S, bool with_diag, bool scatte
         c.diag_buf = c.stage_partials;
     }
     const bool moist = S.stage + 1 == c.n_stages;
-    size_t sm = S.recwin ? recwin_bytes<R>() : 0;
     // the next scatter's scales: vorticity bounds from this kernel, the rest
     // from the step bounds (volume, buoyancy and humidity are those of the
     // step's first par2grid)
@@ -1192,17 +1363,16 @@ static void launch_stage(Ctx& c, const FusedArgs& S, bool with_diag, bool scatte
         Sk.vbound = c.dsc->pbound;
     }
     auto launch = [&](auto kernel) {
-        if (sm) set_smem(kernel, sm);
         prof_begin(c, "stage");
-        kernel<<<g, PB, sm, c.stream>>>(c.P, c.pv, c.n, B, pack, Sk, c.dsc, c.stage_partials, &c.dsc->err);
+        kernel<<<g, PB, 0, c.stream>>>(c.P, c.pv, c.n, B, pack, Sk, c.dsc, c.stage_partials, &c.dsc->err);
         CKL();
         prof_end(c, "stage");
     };
     // the stage kernel may also compute the support vectors of the advanced
     // shapes, which the scatter then reads
     const bool vout = scatter && c.stage_vectors;
-    if (with_diag) vout ? launch(k_stage<true, R, true>) : launch(k_stage<true, R>);
-    else vout ? launch(k_stage<false, R, true>) : launch(k_stage<false, R>);
+    if (with_diag) vout ? launch(k_stage<true, R, true>) : launch(k_stage<true, R, false>);
+    else vout ? launch(k_stage<false, R, true>) : launch(k_stage<false, R, false>);
     if (scatter) {
         prof_begin(c, "stage_p2g");
         // the par2grid of stage + 1: dbuoyg and humg only for the last stage;
@@ -1223,8 +1393,6 @@ void fused_stage(Ctx& c, int stage, bool with_diag) {
     S.last = stage == c.n_stages;
     S.ca = c.ca[stage - 1];
     S.cb = c.cb[stage - 1];
-    S.lg = c.scatter_lg[2];
-    S.recwin = c.stage_recwin;
     // surface fluxes: inside the stage-1 kernel after its diagnostics, or
     // (no diagnostics) by their own kernel before it
     const bool flux = stage == 1 && c.flux_on;

@@ -40,19 +40,10 @@ void autotune(Ctx& c, epic_tuning* out) {
     if (!c.has_parcels || c.n == 0) throw CudaError(EPIC_ERR_STATE, "autotune: no parcels");
     // time the box-ordered paths the steps use (the parcel set is unchanged)
     if (!c.cfg.keep_order) sort_parcels(c);
-    // lane groups of the par2grid scatter (also the stage's par2grid) and of vol2grid
-    int best_p = c.scatter_lg[1], best_v = c.scatter_lg[0];
-    float tp = FLT_MAX, tv = FLT_MAX;
-    for (int lg = 0; lg <= 3; ++lg) {
-        c.scatter_lg[1] = lg;
-        float t = time_ms(c, [&] { par2grid(c, false, true); });
-        if (t < tp) { tp = t; best_p = lg; }
-        c.scatter_lg[0] = lg;
-        t = time_ms(c, [&] { vol2grid(c, false); });
-        if (t < tv) { tv = t; best_v = lg; }
-    }
-    c.scatter_lg[1] = c.scatter_lg[2] = best_p;
-    c.scatter_lg[0] = best_v;
+    // par2grid and vol2grid have one launch shape (a warp takes 32 consecutive
+    // parcels): timed for the report
+    const float tp = time_ms(c, [&] { par2grid(c, false, true); });
+    const float tv = time_ms(c, [&] { vol2grid(c, false); });
     // horizontal FFT path: plane kernel (square grids up to 128), tiled lines, lines of any length,
     // half-plane cluster kernel (square 64 and 128)
     int best_f = c.fft_path;
@@ -67,8 +58,8 @@ void autotune(Ctx& c, epic_tuning* out) {
     par2grid(c, false, true);
     CK(cudaStreamSynchronize(c.stream));
     if (out) {
-        out->lg_par2grid = best_p;
-        out->lg_vol2grid = best_v;
+        out->lg_par2grid = 0;
+        out->lg_vol2grid = 0;
         out->fft_path = best_f;
         out->ms_par2grid = tp;
         out->ms_vol2grid = tv;

@@ -194,9 +194,9 @@ int epic_gpu_init_from_grids(epic_ctx* ctx, const double* vortg, const double* t
                              int32_t zeta_flags[2]);
 
 /* Autotuner (no counterpart in the reference): times the candidate launch
- * shapes of this context on its own parcels and grid -- the lane grouping of
- * the par2grid / vol2grid scatters and the horizontal FFT path -- and keeps
- * the fastest.  Every candidate computes the same result; only calls that
+ * shapes of this context on its own parcels and grid -- the horizontal FFT
+ * path -- and keeps the fastest; par2grid and vol2grid, which have one launch
+ * shape, are timed for the report (lg_par2grid and lg_vol2grid are 0).  Every candidate computes the same result; only calls that
  * leave the state unchanged are timed (par2grid, vol2grid, FFTs into work
  * arrays).  Call after set_parcels / init_state; out may be NULL. */
 typedef struct epic_tuning {

@@ -48,9 +48,8 @@ int epic_gpu_test_reflective_bc(struct epic_ctx* ctx);
  * fftxyp2s / fftxys2p (sta3dfft.f90:134-257). */
 int epic_gpu_test_set_fft_path(struct epic_ctx* ctx, int path);
 
-/* Lane mapping of the scatter kernels: lanes take groups of 2^lg consecutive
- * parcels (lg in 0..5) for vol2grid, par2grid and the fused stage.  Any
- * setting computes the same sums; it only changes the memory access order. */
+/* Lane mapping of the scatter kernels (lg in 0..5 each).  Kept for its callers:
+ * the scatters take 32 consecutive parcels per warp whatever the setting. */
 int epic_gpu_test_set_scatter_groups(struct epic_ctx* ctx, int lg_vol2grid, int lg_par2grid, int lg_stage);
 
 /* Free the second parcel store, as when the device had no room for it: the
@@ -62,8 +61,8 @@ int epic_gpu_test_set_vectors_kernel(struct epic_ctx* ctx, int on);
  * algebra) in FP64 instead of FP32, to measure that part's share of the
  * form's error against FP64. */
 int epic_gpu_test_set_spectral_fp64(struct epic_ctx* ctx, int on);
-/* Stage kernel (split form) gathers from the box's records staged in shared
- * memory (1) or from global memory (0, default); same results. */
+/* Kept for its callers: a window of gather records in shared memory measured
+ * slower and is gone, so the setting changes nothing. */
 int epic_gpu_test_set_stage_window(struct epic_ctx* ctx, int on);
 /* Split-form stage kernel computes the support vectors of the advanced shapes
  * for the next par2grid (1) or a separate kernel does (0, default); same

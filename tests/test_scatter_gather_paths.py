@@ -1,0 +1,88 @@
+"""par2grid, vol2grid and the stage kernel against the oracle where their paths
+change: windows that do not fit the grid, boxes cut by its edge, warps with one
+parcel, parcels of one cell (matrix products) and spread over several (single
+products, shared gather), tails of split children.
+
+Bounds: a fixed-point sum is rounded by 2^-47 of the field's largest value per
+group; a grid point gets less than 2^9 groups and vorticity is divided by a
+volume above 1/16 of the largest: 2^-47 2^9 16 = 6e-11 at most, 1e-12 in the
+root mean square that 2^9 independent roundings give."""
+import numpy as np
+import pytest
+
+from epic_b200 import abi, initial, make_context
+from tests.conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+IDS = list(abi.VORTG) + [abi.TBUOYG, abi.DBUOYG, abi.HUMG, abi.VOLG, abi.NPARG, abi.NSPARG]
+
+
+def state(shape, deform, drop=0, seed=11):
+    """Jittered parcels with axis ratios 1 : deform : deform^2; the last `drop`
+    parcels share the volume of the rest (odd counts)."""
+    s = initial.thermal(*shape, seed=seed)
+    rng = np.random.default_rng(seed)
+    n = s.n
+    q = rng.normal(size=(n, 4))
+    q /= np.linalg.norm(q, axis=1)[:, None]
+    w, x, y, z = q.T
+    R = np.stack([1 - 2 * (y * y + z * z), 2 * (x * y - w * z), 2 * (x * z + w * y),
+                  2 * (x * y + w * z), 1 - 2 * (x * x + z * z), 2 * (y * z - w * x),
+                  2 * (x * z - w * y), 2 * (y * z + w * x), 1 - 2 * (x * x + y * y)], 1).reshape(n, 3, 3)
+    c2 = (0.75 * s.vol / np.pi / deform ** 3) ** (2.0 / 3.0)
+    B = np.einsum("nij,j,nkj->nik", R, np.array([deform ** 4, deform ** 2, 1.0]), R) * c2[:, None, None]
+    s.B = np.stack([B[:, 0, 0], B[:, 0, 1], B[:, 0, 2], B[:, 1, 1], B[:, 1, 2]], 1)
+    s.vor = rng.uniform(-1.0, 1.0, (n, 3))
+    s.hum = np.abs(rng.normal(0.0, 0.01, n)) * (rng.random(n) < 0.5)
+    if drop:
+        for k in ("pos", "vor", "B", "vol", "buoy", "hum"):
+            setattr(s, k, getattr(s, k)[:n - drop].copy())
+    return s
+
+
+# shapes: no window (4 cells), just no window, just one, cut boxes, whole boxes
+@pytest.mark.parametrize("shape", [(4, 4, 2), (10, 6, 3), (12, 8, 5), (18, 10, 7), (16, 16, 16)])
+@pytest.mark.parametrize("deform,drop", [(1.0001, 0), (1.2, 5), (1.9, 31)])
+@pytest.mark.parametrize("keep_order", [0, 1])
+def test_scatter_paths(olib, glib, shape, deform, drop, keep_order):
+    s = state(shape, deform, drop)
+    oc, gc = make_context(s, olib), make_context(s, glib, keep_order=keep_order)
+    if not keep_order:
+        gc.autotune()   # sorts the store by box
+    oc.par2grid(False)
+    gc.par2grid(False)
+    for i in IDS:
+        assert rel_err(gc.get_field(i)[:, :, 1:-1], oc.get_field(i)[:, :, 1:-1]) < 1e-12, abi.FIELD_NAMES[i]
+    oc.vol2grid(True)
+    gc.vol2grid(True)
+    assert rel_err(gc.get_field(abi.VOLG), oc.get_field(abi.VOLG)) < 1e-13
+
+
+@pytest.mark.parametrize("shape,deform,drop", [((12, 8, 5), 1.9, 31), ((16, 16, 16), 1.9, 1), ((16, 16, 16), 1.2, 0),
+                                               ((4, 4, 3), 1.9, 95)])
+@pytest.mark.parametrize("keep_order", [0, 1])
+def test_stage_gather_paths(olib, glib, shape, deform, drop, keep_order):
+    """One RK step (five stages), parcels in container order."""
+    s = state(shape, deform, drop)
+    out = []
+    for lib, kw in ((olib, {}), (glib, dict(keep_order=keep_order))):
+        c = make_context(s, lib, **kw)
+        if lib is glib and not keep_order:
+            c.autotune()
+        t, dt = c.rk_step(0.0)
+        out.append((dt, c.get_parcels()))
+    assert rel_err(out[1][0], out[0][0]) < 1e-10
+    for k, v in out[0][1].items():
+        assert rel_err(out[1][1][k], v) < 1e-10, k
+
+
+def test_scatter_refuses_far_positions(glib):
+    """A position far outside the vertical halo, or an infinite one, is reported
+    and not scattered."""
+    for z in (1.0e12, np.inf):
+        s = state((12, 8, 5), 1.2)
+        s.pos[3, 2] = z
+        gc = make_context(s, glib)
+        for call in (lambda: gc.par2grid(False), lambda: gc.vol2grid(False)):
+            with pytest.raises(abi.EpicError):
+                call()
