@@ -117,6 +117,7 @@ struct Ctx {
     bool vectors_kernel = true;   // support vectors by their own kernel before a scatter that recomputes them
     bool stage_vectors = false;   // split-form stage kernel computes the next par2grid's support vectors
     bool p2g_counted = true;      // the last par2grid scatter counted parcels per cell (nparg, nsparg)
+    bool p2g_moist = true;        // the last par2grid scatter had dbuoyg and humg
     // mixed form with FP64 spectral work (an accuracy experiment; test toggle)
     bool spectral_fp64 = false;
     // the next scatter's bounds are already in pbound (computed by the

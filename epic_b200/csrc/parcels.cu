@@ -32,77 +32,80 @@ EPIC_DEV double fx_inv(const unsigned long long* pbound, int k, int bits) {
     return ldexp(1.0, e - bits);
 }
 
-// z folds (parcel_interpl.f90:237-243, 256-275), per (x, y) column, on the
-// integer sums (exact)
-__global__ void k_p2g_fold(Params P, ScatterFields F, int nf, int* nparg, int* nsparg, long long* count) {
-    long long ncol = (long long)P.nx * P.ny;
-    long long local = 0;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncol;
-         c += (long long)gridDim.x * blockDim.x) {
-        long long t = c * P.nzh + 1;
-        int nz = P.nz;
-        for (int f = 0; f < nf; ++f) {
-            long long* p = reinterpret_cast<long long*>(F.f[f]) + t;
-            p[0] = 2 * p[0];
-            p[nz] = 2 * p[nz];
-            p[1] = p[1] + p[-1];
-            p[nz - 1] = p[nz - 1] + p[nz + 1];
-        }
-        if (nparg) {
-            int* q = nparg + t;
-            int* s = nsparg + t;
-            q[0] += q[-1];
-            q[nz - 1] += q[nz];
-            s[0] += s[-1];
-            s[nz - 1] += s[nz];
-            for (int iz = 0; iz < nz; ++iz) local += q[iz];
-        }
-    }
-    if (nparg) {
-        for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffff, local, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd((unsigned long long*)count, (unsigned long long)local);
-    }
-}
-
-// The integer sums to FP64 on every row; rows 0 .. nz divided by the gridded
-// volume, with the zeta boundary zeroing (parcel_interpl.f90:278-313).
-__global__ void k_p2g_divide(Params P, ScatterFields F, const unsigned long long* pbound, int bits) {
+// After a scatter, per (x, y) column in place: the z folds on the integer sums
+// (exact; parcel_interpl.f90:237-243, 256-275), FP64 values on every row, rows
+// 0 .. nz divided by the gridded volume with the zeta boundary zeroing, and the
+// halo rows of vortg and tbuoyg extrapolated (parcel_interpl.f90:278-319).
+// SET: the scattered fields, 7 = all, 5 = without dbuoyg and humg (they stay
+// zero), 1 = the volume alone (vol2grid).
+//
+// One pass over the fields with a warp per column and z along its lanes, bound
+// by HBM at large grids and by one load-store latency at small ones: the rows
+// that other rows need (the outermost two) are read before any row is written.
+// Fold, division and extrapolation as three kernels with a thread per column in
+// the first and last took 32 us at 48^3 (9 us now) and 92 us at 128^3.
+template <int SET>
+__global__ void __launch_bounds__(PB) k_p2g_tail(Params P, ScatterFields F, int* nparg, int* nsparg, long long* count,
+                                                 const unsigned long long* pbound, int bits) {
+    constexpr int L0 = SET == 1 ? 6 : 0;
+    const int lane = threadIdx.x & 31, nz = P.nz;
+    const int ncol = P.nx * P.ny;
     double inv[7];
 #pragma unroll
-    for (int l = 0; l < 7; ++l) inv[l] = fx_inv(pbound, l, bits);
-    const long long nel = (long long)P.nx * P.ny * P.nzh;
-    PLOOP(nel) {
-        const int iz = (int)(i % P.nzh) - 1;
-        double v[7];
+    for (int l = L0; l < 7; ++l)
+        if (SET != 5 || (l != 3 && l != 4)) inv[l] = fx_inv(pbound, l, bits);
+    long long local = 0;
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < ncol; c += (gridDim.x * blockDim.x) >> 5) {
+        const long long t = (long long)c * P.nzh + 1;
+        long long low[7], high[7];
 #pragma unroll
-        for (int l = 0; l < 7; ++l) v[l] = (double)reinterpret_cast<const long long*>(F.f[l])[i] * inv[l];
-        if (iz >= 0 && iz <= P.nz) {
+        for (int l = L0; l < 7; ++l)
+            if (SET != 5 || (l != 3 && l != 4)) {
+                const long long* p = reinterpret_cast<const long long*>(F.f[l]) + t;
+                low[l] = p[-1];
+                high[l] = p[nz + 1];
+            }
+        __syncwarp();
+        for (int iz = lane - 1; iz <= nz + 1; iz += 32) {
+            const bool inside = iz >= 0 && iz <= nz;
+            double v[7];
 #pragma unroll
-            for (int l = 0; l < 6; ++l) v[l] = v[l] / v[6];
-            if ((iz == 0 && P.zeta_zero[0]) || (iz == P.nz && P.zeta_zero[1])) v[2] = 0.0;
+            for (int l = L0; l < 7; ++l)
+                if (SET != 5 || (l != 3 && l != 4)) {
+                    long long q = reinterpret_cast<const long long*>(F.f[l])[t + iz];
+                    if (iz == 0 || iz == nz) q = 2 * q;
+                    if (iz == 1) q += low[l];
+                    if (iz == nz - 1) q += high[l];
+                    v[l] = (double)q * inv[l];
+                }
+#pragma unroll
+            for (int l = L0; l < 7; ++l)
+                if (SET != 5 || (l != 3 && l != 4)) {
+                    if (l < 6 && inside) v[l] = v[l] / v[6];
+                    if (l == 2 && ((iz == 0 && P.zeta_zero[0]) || (iz == nz && P.zeta_zero[1]))) v[l] = 0.0;
+                    F.f[l][t + iz] = v[l];
+                }
         }
-#pragma unroll
-        for (int l = 0; l < 7; ++l) F.f[l][i] = v[l];
+        __syncwarp();
+        if (SET != 1 && lane < 8) {
+            const int which[4] = {0, 1, 2, 5};
+            double* p = F.f[which[lane >> 1]] + t;
+            if (lane & 1) p[nz + 1] = 2.0 * p[nz] - p[nz - 1];
+            else p[-1] = 2.0 * p[0] - p[1];
+        }
+        if (SET != 1 && nparg) {
+            int* q = nparg + t;
+            int* s = nsparg + t;
+            for (int iz = lane - 1; iz <= nz; iz += 32) local += q[iz];
+            __syncwarp();
+            if (lane == 0) { q[0] += q[-1]; s[0] += s[-1]; }
+            __syncwarp();
+            if (lane == 0) { q[nz - 1] += q[nz]; s[nz - 1] += s[nz]; }
+        }
     }
-}
-
-// vol2grid's integer sums to FP64
-__global__ void k_v2g_convert(long long fsz, double* volg, const unsigned long long* pbound, int bits) {
-    const double inv = fx_inv(pbound, 6, bits);
-    PLOOP(fsz) volg[i] = (double)reinterpret_cast<const long long*>(volg)[i] * inv;
-}
-
-__global__ void k_p2g_halo(Params P, ScatterFields F) {
-    long long ncol = (long long)P.nx * P.ny;
-    PLOOP(ncol) {
-        long long t = i * P.nzh + 1;
-        int nz = P.nz;
-        const int which[4] = {0, 1, 2, 5};
-        for (int q = 0; q < 4; ++q) {
-            double* p = F.f[which[q]] + t;
-            p[-1] = 2.0 * p[0] - p[1];
-            p[nz + 1] = 2.0 * p[nz] - p[nz - 1];
-        }
+    if (SET != 1 && nparg) {
+        for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffff, local, o);
+        if (lane == 0) atomicAdd((unsigned long long*)count, (unsigned long long)local);
     }
 }
 
@@ -118,20 +121,20 @@ void p2g_tail(Ctx& c) {
     ScatterFields F;
     F.f[0] = c.vortg(0); F.f[1] = c.vortg(1); F.f[2] = c.vortg(2);
     F.f[3] = c.dbuoyg(); F.f[4] = c.humg(); F.f[5] = c.tbuoyg(); F.f[6] = c.volg();
-    long long ncol = (long long)P.nx * P.ny;
     // the parcel-count check (parcel_interpl.f90:245-250) where the scatter counted
     const bool counted = c.p2g_counted;
-    k_p2g_fold<<<(int)((ncol + 255) / 256), 256, 0, c.stream>>>(P, F, 7, counted ? c.nparg : nullptr,
-                                                                  c.nsparg, &c.dsc->count);
-    CKL();
+    int* np = counted ? c.nparg : nullptr;
+    auto run = [&](auto kernel) {
+        kernel<<<pgrid((long long)P.nx * P.ny * 32), PB, 0, c.stream>>>(P, F, np, c.nsparg, &c.dsc->count, c.dsc->pbound,
+                                                                       p2g_fx_bits(c));
+        CKL();
+    };
+    if (c.p2g_moist) run(k_p2g_tail<7>);
+    else run(k_p2g_tail<5>);
     if (counted) {
         k_count_check<<<1, 1, 0, c.stream>>>(c.dsc, c.n);
         CKL();
     }
-    k_p2g_divide<<<pgrid((long long)P.nx * P.ny * P.nzh), PB, 0, c.stream>>>(P, F, c.dsc->pbound, p2g_fx_bits(c));
-    CKL();
-    k_p2g_halo<<<(int)((ncol + 255) / 256), 256, 0, c.stream>>>(P, F);
-    CKL();
 }
 
 void par2grid(Ctx& c, bool reuse, bool store_vectors, bool moist) {
@@ -145,11 +148,9 @@ void vol2grid(Ctx& c, bool reuse) {
     const Params& P = c.P;
     scatter_v2g(c, reuse);
     ScatterFields F;
-    F.f[0] = c.volg();
-    long long ncol = (long long)P.nx * P.ny;
-    k_p2g_fold<<<(int)((ncol + 255) / 256), 256, 0, c.stream>>>(P, F, 1, nullptr, nullptr, nullptr);
-    CKL();
-    k_v2g_convert<<<pgrid(P.fsz), PB, 0, c.stream>>>(P.fsz, c.volg(), c.dsc->pbound, p2g_fx_bits(c));
+    F.f[6] = c.volg();
+    k_p2g_tail<1><<<pgrid((long long)P.nx * P.ny * 32), PB, 0, c.stream>>>(P, F, nullptr, nullptr, nullptr, c.dsc->pbound,
+                                                                            p2g_fx_bits(c));
     CKL();
 }
 
@@ -765,7 +766,7 @@ __global__ void k_split_flag(Params P, PView pv, long long n, int* flag, unsigne
     }
     vmax = isnan(vmax) ? INFINITY : vmax;
     for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffff, vmax, o));
-    if ((threadIdx.x & 31) == 0 && vmax > 0.0) atomicMax(vbound, (unsigned long long)__double_as_longlong(vmax));
+    if ((threadIdx.x & 31) == 0 && vmax > 0.0) atomic_max_nonneg(vbound, vmax);
 }
 
 __global__ void k_split_apply(Params P, PView pv, long long n, const int* flag, const int* offs, long long* label,

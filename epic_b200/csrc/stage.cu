@@ -1296,12 +1296,14 @@ static void launch_scatter(Ctx& c, const Fields7& F, bool reuse, bool store, boo
 template <class R>
 static void launch_p2g(Ctx& c, bool moist, bool reuse, bool store, bool count) {
     c.p2g_counted = count;
+    c.p2g_moist = moist;
     if (moist) launch_scatter<7, R>(c, fields7(c), reuse, store, count);
     else launch_scatter<5, R>(c, fields7(c), reuse, store, count);
 }
 
 void scatter_p2g(Ctx& c, bool reuse, bool store, bool moist) {
     zero_p2g_fields(c);
+    c.p2g_moist = true;
     if (c.n == 0) return;
     prof_begin(c, "p2g");
     if (c.pv.mixed) launch_p2g<float>(c, moist, reuse, store, true);
