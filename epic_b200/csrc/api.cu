@@ -354,6 +354,7 @@ static void free_ctx(Ctx& c) {
     if (c.scratch) cudaFree(c.scratch);
     if (c.scratch2) cudaFree(c.scratch2);
     if (c.hsc) cudaFreeHost(c.hsc);
+    if (c.spread_ev) cudaEventDestroy(c.spread_ev);
     if (c.stream) cudaStreamDestroy(c.stream);
     c.stream = nullptr;
 }
@@ -432,6 +433,7 @@ int epic_gpu_create(const epic_cfg* cfg, epic_ctx** out) {
         CK(cudaMalloc(&c.dsc, sizeof(StepScalars)));
         CK(cudaMemsetAsync(c.dsc, 0, sizeof(StepScalars), c.stream));
         CK(cudaMallocHost(&c.hsc, sizeof(StepScalars)));
+        CK(cudaEventCreateWithFlags(&c.spread_ev, cudaEventDisableTiming));
         CK(cudaMalloc(&c.partials, sizeof(double) * 148 * 8 * 64));
         CK(cudaMalloc(&c.stage_partials, sizeof(double) * 16 * (size_t)stage_grid_max(P, c.cap)));
         // gather records: 16 values per grid point (FP32 in the mixed form)
@@ -702,8 +704,13 @@ static double rk_step(Ctx& c, double& t, double* pstats, double* fstats) {
     // scatter bounds its own values)
     p2g_step_bounds(c);
     c.p2g_bound_ready = true;
+    c.spread = false;
+    c.count_spread = true;
     par2grid(c, t > c.cfg.t_initial, true, c.n_stages == 1);
+    c.count_spread = false;
     c.p2g_bound_ready = false;
+    CK(cudaMemcpyAsync(&c.hsc->spread, &c.dsc->spread, sizeof(c.dsc->spread), cudaMemcpyDeviceToHost, c.stream));
+    CK(cudaEventRecord(c.spread_ev, c.stream));
     c.pstep_valid = !c.flux_on;
     prof_begin(c, "vor2vel");
     vor2vel(c);
@@ -715,6 +722,9 @@ static double rk_step(Ctx& c, double& t, double* pstats, double* fstats) {
     time_step_reduce(c, flux_dt_bound(c));
     prof_end(c, "timestep");
     if (fstats) field_diagnostics(c, fstats);
+    // known by now: the inversion queued behind the count keeps the device busy
+    CK(cudaEventSynchronize(c.spread_ev));
+    c.spread = c.hsc->spread > (unsigned long long)c.n / 4;
     for (int s = 1; s <= c.n_stages; ++s) {
         if (s > 1) {
             prof_begin(c, "vor2vel");
@@ -737,6 +747,7 @@ static double rk_step(Ctx& c, double& t, double* pstats, double* fstats) {
         prof_end(c, "damping");
     }
     c.pstep_valid = false;
+    c.spread = false;
     if (pstats) finish_parcel_diag(c, pstats);
     double dt = 0.0;
     CK(cudaMemcpyAsync(&dt, &c.dsc->dt, sizeof(double), cudaMemcpyDeviceToHost, c.stream));

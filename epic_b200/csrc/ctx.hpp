@@ -78,6 +78,8 @@ struct StepScalars {
     // not change between its stages): 0.25 V |b|, 0.25 V |h|,
     // 0.25 V (|b| + glat max(h, 0)) (above |tbuoyg|'s values), 0.25 V
     unsigned long long pstep[4];
+    // parcels with support points in several cells, at the step's first par2grid
+    unsigned long long spread;
     // 0.25 V over the parcels after the split test (vol2grid of the corrections)
     unsigned long long vbound;
 };
@@ -129,6 +131,13 @@ struct Ctx {
     // StepScalars::pstep holds this step's bounds (set by rk_step's first
     // par2grid when the stages change no volume, buoyancy or humidity)
     bool pstep_valid = false;
+    // Set during the stages of a step: a deformed flow, in which at the step's
+    // first par2grid more than a quarter of the parcels had support points in several cells.  Chooses between kernels that
+    // compute the same sums (rounding aside), each the faster one on its side: at
+    // a quarter the stage kernels of a deformed 64^3 flow cost the same.
+    bool spread = false;
+    bool count_spread = false;    // the next par2grid scatter counts them
+    cudaEvent_t spread_ev = nullptr;
     // labels (cfg.labels): label and dilution per parcel, capacity cap
     long long* label = nullptr;
     double* dil = nullptr;

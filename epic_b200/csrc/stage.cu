@@ -414,7 +414,8 @@ EPIC_DEV void support_point(const double* pos, const double* eta, const double* 
 }
 // The points lie on an ellipse in the order 0..3; starting the merge at a
 // point whose predecessor (cyclically) is in another cell also merges a run
-// that wraps from point 3 to point 0.
+// that wraps from point 3 to point 0.  NONE: all points in one cell.
+template <int NONE = 0>
 EPIC_DEV int merge_start(const Params& P, const double* pos, const double* eta, const double* tau) {
     int c[4][3];
 #pragma unroll
@@ -429,7 +430,7 @@ EPIC_DEV int merge_start(const Params& P, const double* pos, const double* eta, 
         const int q = (p + 3) & 3;
         if (c[p][0] != c[q][0] || c[p][1] != c[q][1] || c[p][2] != c[q][2]) return p;
     }
-    return 0;
+    return NONE;
 }
 
 // D += A B on the FP64 tensor path: A 8 x 4 (lane: row lane / 4, column
@@ -705,8 +706,9 @@ EPIC_DEV void vectors(const PView& pv, long long i, bool reuse, bool store, R* e
 // a warp takes 32 consecutive parcels, one per lane.
 template <int NF, class R, bool VEC = true>
 EPIC_DEV void scatter_parcels(const Params& P, const PView& pv, long long q0, long long q1, const WinShared<NF>* ws,
-                              unsigned* acc, WarpRows<NF>* rows, const Fields7& F, int* nparg, int* nsparg, bool reuse,
-                              bool store, unsigned* err) {
+                              unsigned* acc, WarpRows<NF>* rows, const Fields7& F, int* nparg, int* nsparg,
+                              unsigned long long* spread, bool reuse, bool store, unsigned* err) {
+    unsigned several = 0;   // parcels of this lane with points in several cells
     const Window W = ws->W;
     const int lane = threadIdx.x & 31;
     for (long long ib = q0 + (threadIdx.x & ~31); ib < q1; ib += blockDim.x) {
@@ -735,6 +737,7 @@ EPIC_DEV void scatter_parcels(const Params& P, const PView& pv, long long q0, lo
             const double td[3] = {(double)tau[0], (double)tau[1], (double)tau[2]};
             pts.set(P, pos, ed, td);
             same = point_groups(pts);
+            several += (same & 15) != 15;
             if (pts.z_near()) todo = 15;
             else set_err(err, ERRB_ZRANGE);
         }
@@ -774,6 +777,10 @@ EPIC_DEV void scatter_parcels(const Params& P, const PView& pv, long long q0, lo
                 scatter_products<NF, R>(P, acc, F, code, flip, w, v);
             }
         }
+    }
+    if (spread) {
+        several = __reduce_add_sync(0xffffffffu, several);
+        if (lane == 0 && several) atomicAdd(spread, (unsigned long long)several);
     }
 }
 
@@ -856,7 +863,8 @@ template <int NF, class R, bool VEC>
 __global__ void __launch_bounds__(PB, NF == 1 ? 3 : 2) k_scatter(Params P, PView pv, long long n, Boxes B,
                                                                  const __grid_constant__ Fields7 F,
                                                                  const unsigned long long* pbound, int* nparg,
-                                                                 int* nsparg, int reuse, int store, unsigned* err) {
+                                                                 int* nsparg, unsigned long long* spread, int reuse,
+                                                                 int store, unsigned* err) {
     extern __shared__ __align__(16) unsigned acc[];
     __shared__ WinShared<NF> ws;
     constexpr size_t wbytes = (win_bytes<NF>() + 15) & ~(size_t)15;
@@ -880,7 +888,8 @@ __global__ void __launch_bounds__(PB, NF == 1 ? 3 : 2) k_scatter(Params P, PView
         win_zero<NF>(acc, ws.W);
         __syncthreads();
         if constexpr (NF == 1) scatter_volumes<R, VEC>(P, pv, q0, q1, &ws, acc, F, reuse != 0, store != 0, err);
-        else scatter_parcels<NF, R, VEC>(P, pv, q0, q1, &ws, acc, rows, F, nparg, nsparg, reuse != 0, store != 0, err);
+        else scatter_parcels<NF, R, VEC>(P, pv, q0, q1, &ws, acc, rows, F, nparg, nsparg, spread, reuse != 0,
+                                         store != 0, err);
         __syncthreads();
         win_flush<NF, R>(P, acc, ws.W, F);
         __syncthreads();
@@ -928,6 +937,14 @@ __global__ void k_pack_gather(GatherFields G, R* pack, long long fsz) {
 // over a parcel's runs and their 8 corners of w / 4 times field l (the point
 // weight 1/4), from the records of 16 values per grid point.
 //
+// Staging rows of a warp for gather_shared: a run's weights and cell columns,
+// then a parcel's 16 sums (rows of 10 and 18 doubles: conflict-free 16-byte
+// accesses of a quarter warp).
+union alignas(16) GatherRows {
+    struct { double w[8]; int col[4]; } run[32];
+    double sum[32][GREC + 2];
+};
+
 // One parcel per lane: every lane reads the records of its own cells.  A load
 // instruction of the warp takes a pass through L1 for each cell among the lanes,
 // few where neighbours in the store share cells.  Support points in the cell of
@@ -991,6 +1008,84 @@ EPIC_DEV bool gather_own(const Params& P, const R* __restrict__ pack, const doub
     return gather_tri<R>(P, pack, cur, g) && ok;
 }
 
+// The warp's runs one after another (plain form), 8 lanes per run: a lane reads
+// one 16-byte word of the run's records, so that a record is one 128-byte access
+// and a load instruction touches 4 records whatever the cells.  For parcels
+// spread over several cells each, where gather_own is bound by its L1 passes (up
+// to 32 per load): stage kernel 0.70 -> 0.52 ms on 2.4M deformed parcels.  The
+// mixed form's records are half as long and gained nothing (9.2 -> 9.8 ms).
+//
+// Not inlined: its registers (the sums of 8 sets) would push the state of
+// gather_own's callers out.  The sums are left in rows->sum.
+__device__ __noinline__ bool gather_shared(int nx, int ny, int nz, const double* __restrict__ pack, Points pts, bool valid,
+                                           GatherRows* rows) {
+    const int same = point_groups(pts), nzh = nz + 3;
+    constexpr int NS = 8;   // sets of 4 runs
+    const int lane = threadIdx.x & 31, part = lane & 7, mine = lane >> 3;
+    double acc[NS][2];
+#pragma unroll
+    for (int s = 0; s < NS; ++s) acc[s][0] = acc[s][1] = 0.0;
+    bool ok = pts.z_near();
+    int todo = valid && ok ? 15 : 0;
+    while (__any_sync(0xffffffffu, todo != 0)) {
+        bool active = todo != 0;
+        __syncwarp();   // the rows of the previous runs are read
+        if (active) {
+            const int m = same >> (4 * (__ffs(todo) - 1)) & 15;
+            todo &= ~m;
+            Run run;
+            run.set(pts, m);
+            if (run.c[2] < -1 || run.c[2] > nz) {
+                ok = active = false;
+            } else {
+                double w[8];
+                run.weights(w);
+                double2* wr = reinterpret_cast<double2*>(rows->run[lane].w);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) wr[k] = make_double2(0.25 * w[2 * k], 0.25 * w[2 * k + 1]);
+                // the records of the lower corners of the cell's 4 columns
+                const int x0 = wrap_to(run.c[0], nx), y0 = wrap_to(run.c[1], ny), z = run.c[2] + 1;
+                const int x1 = x0 + 1 == nx ? 0 : x0 + 1, y1 = y0 + 1 == ny ? 0 : y0 + 1;
+                *reinterpret_cast<int4*>(rows->run[lane].col) =
+                    make_int4((x0 * ny + y0) * nzh + z, (x0 * ny + y1) * nzh + z, (x1 * ny + y0) * nzh + z,
+                              (x1 * ny + y1) * nzh + z);
+            }
+        }
+        const unsigned act = __ballot_sync(0xffffffffu, active);
+        __syncwarp();
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const int r = 4 * s + mine;
+            if (act >> r & 1) {
+                const int4 col = *reinterpret_cast<const int4*>(rows->run[r].col);
+                const double2* q = reinterpret_cast<const double2*>(pack) + part;
+                const int c4[4] = {col.x, col.y, col.z, col.w};
+#pragma unroll
+                for (int k0 = 0; k0 < 8; k0 += 4) {   // 4 loads in flight
+                    double2 v[4];
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) v[k] = __ldg(q + ((long long)c4[(k0 + k) >> 1] + (k & 1)) * (GREC / 2));
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const double w = rows->run[r].w[k0 + k];
+                        acc[s][0] = fma(w, v[k].x, acc[s][0]);
+                        acc[s][1] = fma(w, v[k].y, acc[s][1]);
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < NS; ++s)
+        *reinterpret_cast<double2*>(&rows->sum[4 * s + mine][2 * part]) = make_double2(acc[s][0], acc[s][1]);
+    __syncwarp();
+    return ok;
+}
+// Parcels of a warp with points in several cells above which gather_shared is
+// used (2, 8 and 16 measured alike within 3%).
+constexpr int SPREAD_MAX = 8;
+
 // get_dBdt (parcel_ellipsoid.f90:466-507) in the attribute type.
 template <class R>
 EPIC_DEV void dBdt_r(const R* s, const R* b, R B33, R* o) {
@@ -1003,7 +1098,8 @@ EPIC_DEV void dBdt_r(const R* s, const R* b, R B33, R* o) {
 }
 
 
-template <bool DIAG, class R, bool VOUT>
+// SHARED (plain form): warps with parcels in several cells use gather_shared.
+template <bool DIAG, class R, bool VOUT, bool SHARED>
 __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long n, Boxes B, const R* pack,
                                                   FusedArgs S, const StepScalars* sc, double* partials,
                                                   unsigned* err) {
@@ -1024,10 +1120,17 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
 #define DACC(k) dacc[(k) * PB]
     const double dt = sc->dt;
     const Range Rg = cta_range(P, pv, B, n);
+    extern __shared__ __align__(16) unsigned char stage_smem[];
+    GatherRows* grows = reinterpret_cast<GatherRows*>(stage_smem) + (threadIdx.x >> 5);
     {
         const long long q0 = Rg.r0, q1 = Rg.r1;
-        // grid2par + dB/dt + LS-RK update
-        for (long long i = q0 + threadIdx.x; i < q1; i += blockDim.x) {
+        // grid2par + dB/dt + LS-RK update, 32 consecutive parcels per warp
+        for (long long i0 = q0 + (threadIdx.x & ~31); i0 < q1; i0 += blockDim.x) {
+            const bool valid = i0 + (threadIdx.x & 31) < q1;
+            // lanes past the end leave, or (SHARED: the warp gathers together)
+            // repeat the last parcel and write nothing
+            if (!SHARED && !valid) break;
+            const long long i = valid ? i0 + (threadIdx.x & 31) : q1 - 1;
             // bring the next parcel's attribute lines into L2 (one lane per 128-byte line)
             if ((threadIdx.x & 15) == 0 && i + blockDim.x < q1) {
                 const long long j = i + blockDim.x;
@@ -1043,7 +1146,9 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
             }
             double pos[3] = {a64<R>(pv, A_X, i), a64<R>(pv, A_Y, i), a64<R>(pv, A_Z, i)};
             // the attributes of the update are loaded before the gathers, so
-            // that their latency overlaps the interpolation
+            // that their latency overlaps the interpolation (SHARED: after, as
+            // the sums of gather_shared need the registers)
+            constexpr bool LATE = SHARED;
             R b[5], vor[3];
             double vol;
             auto load_state = [&]() {
@@ -1053,7 +1158,7 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
 #pragma unroll
                 for (int k = 0; k < 3; ++k) vor[k] = aR<R>(pv, A_VX + k, i);
             };
-            load_state();
+            if constexpr (!LATE) load_state();
             // the LS-RK accumulators: the mixed form loads them before the
             // gathers (their latency overlaps the interpolation); the FP64
             // form after them (fewer live registers, no spills)
@@ -1077,8 +1182,30 @@ __global__ void __launch_bounds__(PB, SB) k_stage(Params P, PView pv, long long 
                 for (int k = 0; k < 3; ++k) { eta[k] = aR<R>(pv, A_ETA0 + k, i); tau[k] = aR<R>(pv, A_TAU0 + k, i); }
                 const double ed[3] = {(double)eta[0], (double)eta[1], (double)eta[2]};
                 const double td[3] = {(double)tau[0], (double)tau[1], (double)tau[2]};
-                if (!gather_own<R>(P, pack, pos, ed, td, merge_start(P, pos, ed, td), g)) set_err(err, ERRB_ZRANGE);
+                bool ok;
+                if constexpr (!SHARED) {
+                    ok = gather_own<R>(P, pack, pos, ed, td, merge_start(P, pos, ed, td), g);
+                } else {
+                    const int s0 = merge_start<-1>(P, pos, ed, td);
+                    if (__popc(__ballot_sync(0xffffffffu, valid && s0 >= 0)) > SPREAD_MAX) {
+                        Points pts;
+                        pts.set(P, pos, ed, td);
+                        ok = gather_shared(P.nx, P.ny, P.nz, pack, pts, valid, grows);
+#pragma unroll
+                        for (int l = 0; l < 14; l += 2) {
+                            const double2 v = *reinterpret_cast<const double2*>(&grows->sum[threadIdx.x & 31][l]);
+                            g[l] = v.x;
+                            g[l + 1] = v.y;
+                        }
+                        __syncwarp();
+                    } else {
+                        ok = gather_own<R>(P, pack, pos, ed, td, max(s0, 0), g);
+                    }
+                }
+                if (!ok) set_err(err, ERRB_ZRANGE);
             }
+            if (SHARED && !valid) continue;
+            if constexpr (LATE) load_state();
             if constexpr (!Form<R>::mixed) load_accumulators();
             double dp[3];
             R dv[3];
@@ -1284,8 +1411,8 @@ static void launch_scatter(Ctx& c, const Fields7& F, bool reuse, bool store, boo
     int* nsp = count ? c.nsparg : nullptr;
     auto run = [&](auto kernel) {
         set_smem(kernel, sm);
-        kernel<<<sgrid(c, B), PB, sm, c.stream>>>(c.P, c.pv, c.n, B, F, c.dsc->pbound, np, nsp, reuse, store,
-                                                  &c.dsc->err);
+        kernel<<<sgrid(c, B), PB, sm, c.stream>>>(c.P, c.pv, c.n, B, F, c.dsc->pbound, np, nsp,
+                                                  c.count_spread ? &c.dsc->spread : nullptr, reuse, store, &c.dsc->err);
         CKL();
     };
     if (reuse) run(k_scatter<NF, R, false>);
@@ -1325,7 +1452,8 @@ void scatter_v2g(Ctx& c, bool reuse) {
 // The scales of the step's first par2grid and the step bounds (pstep) that
 // the later stages' scatters take with their vorticity bounds.
 void p2g_step_bounds(Ctx& c) {
-    CK(cudaMemsetAsync(c.dsc->pbound, 0, sizeof(c.dsc->pbound) + sizeof(c.dsc->pstep), c.stream));
+    CK(cudaMemsetAsync(c.dsc->pbound, 0, 
+                       sizeof(c.dsc->pbound) + sizeof(c.dsc->pstep) + sizeof(c.dsc->spread), c.stream));
     if (c.n == 0) return;
     if (c.pv.mixed) k_p2g_bounds<7, float, true><<<pgrid(c.n), PB, 0, c.stream>>>(c.P, c.pv, c.n, c.dsc->pbound, c.dsc->pstep);
     else k_p2g_bounds<7, double, true><<<pgrid(c.n), PB, 0, c.stream>>>(c.P, c.pv, c.n, c.dsc->pbound, c.dsc->pstep);
@@ -1364,17 +1492,28 @@ static void launch_stage(Ctx& c, const FusedArgs& S, bool with_diag, bool scatte
         CK(cudaMemcpyAsync(&c.dsc->pbound[3], c.dsc->pstep, sizeof(c.dsc->pstep), cudaMemcpyDeviceToDevice, c.stream));
         Sk.vbound = c.dsc->pbound;
     }
+    const bool shared = !Form<R>::mixed && c.spread;
     auto launch = [&](auto kernel) {
+        const size_t sm = shared ? sizeof(GatherRows) * (PB / 32) : 0;
+        if (sm) set_smem(kernel, sm);
         prof_begin(c, "stage");
-        kernel<<<g, PB, 0, c.stream>>>(c.P, c.pv, c.n, B, pack, Sk, c.dsc, c.stage_partials, &c.dsc->err);
+        kernel<<<g, PB, sm, c.stream>>>(c.P, c.pv, c.n, B, pack, Sk, c.dsc, c.stage_partials, &c.dsc->err);
         CKL();
         prof_end(c, "stage");
     };
     // the stage kernel may also compute the support vectors of the advanced
     // shapes, which the scatter then reads
     const bool vout = scatter && c.stage_vectors;
-    if (with_diag) vout ? launch(k_stage<true, R, true>) : launch(k_stage<true, R, false>);
-    else vout ? launch(k_stage<false, R, true>) : launch(k_stage<false, R, false>);
+    if constexpr (!Form<R>::mixed) {
+        if (shared) {
+            if (with_diag) vout ? launch(k_stage<true, R, true, true>) : launch(k_stage<true, R, false, true>);
+            else vout ? launch(k_stage<false, R, true, true>) : launch(k_stage<false, R, false, true>);
+        }
+    }
+    if (!shared) {
+        if (with_diag) vout ? launch(k_stage<true, R, true, false>) : launch(k_stage<true, R, false, false>);
+        else vout ? launch(k_stage<false, R, true, false>) : launch(k_stage<false, R, false, false>);
+    }
     if (scatter) {
         prof_begin(c, "stage_p2g");
         // the par2grid of stage + 1: dbuoyg and humg only for the last stage;
