@@ -132,9 +132,13 @@ enum ErrBits {
 
 EPIC_DEV void set_err(unsigned* err, unsigned bit) { atomicOr(err, bit); }
 
-// Monotone encoding of a non-negative double for atomicMax on 64-bit ints.
+// Maximum of non-negative doubles through their ordered bits.  A value that does
+// not raise the maximum, nearly every one of a launch's, is dropped by a read of
+// the (possibly older, so smaller) maximum: atomics on one address serialise, and
+// one per warp took 30 us of a step's first bound pass on 900,000 parcels.
 EPIC_DEV void atomic_max_nonneg(unsigned long long* addr, double v) {
-    atomicMax(addr, (unsigned long long)__double_as_longlong(v));
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+    if (bits > __ldcg(addr)) atomicMax(addr, bits);
 }
 
 }  // namespace epic

@@ -635,14 +635,13 @@ EPIC_DEV void load_values(const Params& P, const PView& pv, long long i, double 
 // a non-negative double; a NaN counts as +inf), into pbound, which the caller
 // cleared: the fixed-point scales of the scatter that follows.  STEP also
 // records the step bounds (StepScalars::pstep) for the later stages' scatters.
-EPIC_DEV unsigned long long max_bits(double a) { return (unsigned long long)__double_as_longlong(a); }
 EPIC_DEV double nan_inf(double a) { return isnan(a) ? INFINITY : a; }
 EPIC_DEV double keep_max(double m, double a) { return (a > m || a != a) ? a : m; }
 // warp maximum, then one atomic per warp
 EPIC_DEV void warp_max_to(unsigned long long* dst, double v) {
     v = nan_inf(v);
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffff, v, o));
-    if ((threadIdx.x & 31) == 0 && v > 0.0) atomicMax(dst, max_bits(v));
+    if ((threadIdx.x & 31) == 0 && v > 0.0) atomic_max_nonneg(dst, v);
 }
 template <int NF, class R, bool STEP>
 __global__ void __launch_bounds__(PB) k_p2g_bounds(Params P, PView pv, long long n, unsigned long long* pbound,
