@@ -10,9 +10,8 @@
 //
 // The scratch holds NOALLOC_MAX_BLOCKS x 4 doubles (128 KiB) plus 8 doubles
 // for the final correction; every GPU that loads the library keeps it until
-// the process exits.  The number of blocks grows with the parcel count (one
-// block per NOALLOC_CHUNK parcels), so the largest accepted parcel count is
-// NOALLOC_MAX_BLOCKS * NOALLOC_CHUNK = 67,108,864.  All calls share the one
+// the process exits.  The largest accepted parcel count is NOALLOC_MAX_BLOCKS *
+// NOALLOC_CHUNK = 67,108,864.  All calls share the one
 // array: two calls whose kernels overlap on the GPU (different streams, no
 // ordering between them) race on it and give wrong results.
 #include "../../include/epic_gpu.h"
@@ -26,7 +25,8 @@ namespace {
 
 constexpr int NOALLOC_THREADS = 256;
 constexpr int NOALLOC_MAX_BLOCKS = 4096;
-constexpr long long NOALLOC_CHUNK = 16384;   // parcels per block (64 per thread)
+constexpr long long NOALLOC_CHUNK = 16384;   // parcels per partial at the largest count
+constexpr int NOALLOC_BLOCKS = 148 * 4;      // partials written
 
 // Block partials (4 per block: sum V, sum V wx, sum V wy, sum V wz) followed
 // by the final correction dvor[3].
@@ -58,21 +58,10 @@ int scratch_for_current_device(cudaStream_t st, double** out) {
     return EPIC_OK;
 }
 
-// Pass 1: each block reduces its chunk in a fixed order and writes its slot.
-__global__ void __launch_bounds__(NOALLOC_THREADS) k_na_partials(long long n, const double* vol, const double* vor,
-                                                                double* scratch) {
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    long long b0 = (long long)blockIdx.x * NOALLOC_CHUNK;
-    long long b1 = min(b0 + NOALLOC_CHUNK, n);
-    for (long long i = b0 + threadIdx.x; i < b1; i += NOALLOC_THREADS) {
-        double v = vol[i];
-        acc[0] += v;
-        acc[1] += vor[3 * i] * v;
-        acc[2] += vor[3 * i + 1] * v;
-        acc[3] += vor[3 * i + 2] * v;
-    }
+// Fixed-order sum over the block of 4 values per thread, in every thread.
+__device__ __forceinline__ void block_sum4(double (&acc)[4]) {
     __shared__ double red[NOALLOC_THREADS / 32][4];
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         double v = acc[k];
@@ -80,30 +69,50 @@ __global__ void __launch_bounds__(NOALLOC_THREADS) k_na_partials(long long n, co
         if (l == 0) red[w][k] = v;
     }
     __syncthreads();
-    if (threadIdx.x < 4) {
-        double v = 0.0;
-        for (int q = 0; q < NOALLOC_THREADS / 32; ++q) v += red[q][threadIdx.x];
-        scratch[blockIdx.x * 4 + threadIdx.x] = v;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        acc[k] = 0.0;
+        for (int q = 0; q < NOALLOC_THREADS / 32; ++q) acc[k] += red[q][k];
     }
 }
 
-// Pass 2: fixed-order sum of the partials -> dvor = mean vorticity - vor_bar
-// (parcel_correction.f90:117-124).
-__global__ void k_na_final(int nb, double b0, double b1, double b2, double* scratch) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = 0; b < nb; ++b)
-        for (int k = 0; k < 4; ++k) s[k] += scratch[b * 4 + k];
-    double* dvor = scratch + NOALLOC_MAX_BLOCKS * 4;
-    dvor[0] = s[1] / s[0] - b0;
-    dvor[1] = s[2] / s[0] - b1;
-    dvor[2] = s[3] / s[0] - b2;
+// Pass 1: each block reduces its chunk in a fixed order and writes its slot.
+__global__ void __launch_bounds__(NOALLOC_THREADS) k_na_partials(long long n, long long chunk, const double* vol,
+                                                                const double* vor, double* scratch) {
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const long long b0 = (long long)blockIdx.x * chunk, b1 = min(b0 + chunk, n);
+#pragma unroll 4
+    for (long long i = b0 + threadIdx.x; i < b1; i += NOALLOC_THREADS) {
+        const double v = vol[i];
+        acc[0] += v;
+        acc[1] += vor[3 * i] * v;
+        acc[2] += vor[3 * i + 1] * v;
+        acc[3] += vor[3 * i + 2] * v;
+    }
+    block_sum4(acc);
+    if (threadIdx.x < 4)
+        scratch[blockIdx.x * 4 + threadIdx.x] = threadIdx.x == 0 ? acc[0] : threadIdx.x == 1 ? acc[1] : threadIdx.x == 2 ? acc[2] : acc[3];
 }
 
-// Pass 3: subtract the correction (parcel_correction.f90:126-133).
-__global__ void k_na_apply(long long n, double* vor, const double* scratch) {
-    const double* dvor = scratch + NOALLOC_MAX_BLOCKS * 4;
-    double d0 = dvor[0], d1 = dvor[1], d2 = dvor[2];
+// Pass 2: every block sums the partials in the same fixed order, dvor = mean
+// vorticity - vor_bar (parcel_correction.f90:117-124), and subtracts it from
+// its parcels (:126-133); block 0 leaves dvor in the scratch.  At most
+// NOALLOC_BLOCKS partials, 19 KiB from L2 per block: cheaper than a launch of
+// its own whose one thread added them.
+__global__ void __launch_bounds__(NOALLOC_THREADS) k_na_apply(long long n, int nb, double b0, double b1, double b2,
+                                                              double* vor, double* scratch) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < nb; b += NOALLOC_THREADS)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[k] += scratch[b * 4 + k];
+    block_sum4(s);
+    const double d0 = s[1] / s[0] - b0, d1 = s[2] / s[0] - b1, d2 = s[3] / s[0] - b2;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        double* dvor = scratch + NOALLOC_MAX_BLOCKS * 4;
+        dvor[0] = d0;
+        dvor[1] = d1;
+        dvor[2] = d2;
+    }
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         vor[3 * i] = vor[3 * i] - d0;
         vor[3 * i + 1] = vor[3 * i + 1] - d1;
@@ -121,11 +130,13 @@ extern "C" int epic_gpu_apply_vortcor_noalloc(int64_t n, const double* vol, doub
     double* scratch = nullptr;
     int rc = scratch_for_current_device(st, &scratch);
     if (rc != EPIC_OK) return rc;
-    int nb = (int)((n + NOALLOC_CHUNK - 1) / NOALLOC_CHUNK);
-    k_na_partials<<<nb, NOALLOC_THREADS, 0, st>>>(n, vol, vor, scratch);
-    k_na_final<<<1, 32, 0, st>>>(nb, vor_bar[0], vor_bar[1], vor_bar[2], scratch);
-    int ab = (int)std::min<long long>((n + 255) / 256, 148LL * 16);
-    k_na_apply<<<ab, 256, 0, st>>>(n, vor, scratch);
+    // 4 parcels per thread where that fills the device no more than 4 times over
+    // (one block per 16384 left 135 of the SMs idle at 200,000 parcels)
+    const long long chunk = std::max<long long>(4 * NOALLOC_THREADS, (n + NOALLOC_BLOCKS - 1) / NOALLOC_BLOCKS);
+    const int nb = (int)((n + chunk - 1) / chunk);
+    k_na_partials<<<nb, NOALLOC_THREADS, 0, st>>>(n, chunk, vol, vor, scratch);
+    const int ab = (int)std::min<long long>((n + NOALLOC_THREADS - 1) / NOALLOC_THREADS, 148LL * 16);
+    k_na_apply<<<ab, NOALLOC_THREADS, 0, st>>>(n, nb, vor_bar[0], vor_bar[1], vor_bar[2], vor, scratch);
     if (cudaGetLastError() != cudaSuccess) return EPIC_ERR_CUDA;
     if (dvor_out) {
         if (cudaMemcpyAsync(dvor_out, scratch + NOALLOC_MAX_BLOCKS * 4, 3 * sizeof(double), cudaMemcpyDeviceToHost,
