@@ -1489,13 +1489,38 @@ struct MPtr8 {
     double* p[8];
 };
 
-// vel2vgrad tail (inversion.f90:308-312) over all rows incl. the halo rows.
-__global__ void k_velgrad_fill(MPtr8 vg, Ptr8 vort, long long fsz) {
+// vel2vgrad tail (inversion.f90:302-312): the halo rows of the velocity and of
+// the transformed gradients (extrapolated, or antisymmetric where the field is
+// odd in z at the boundaries), and the other three gradients from the vorticity on
+// all rows.  One pass: a halo element needs rows that no thread of it writes.
+struct VelTail {
+    double* vel[3];
+    double* vg[8];
+    const double* vort[3];
+};
+__global__ void k_velgrad_fill(VelTail A, int nzh, long long fsz) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < fsz;
          i += (long long)gridDim.x * blockDim.x) {
-        vg.p[I_DUDZ][i] = vg.p[I_DWDX][i] + vort.p[1][i];
-        vg.p[I_DVDX][i] = vg.p[I_DUDY][i] + vort.p[2][i];
-        vg.p[I_DVDZ][i] = vg.p[I_DWDY][i] - vort.p[0][i];
+        const int r = (int)((unsigned)i % (unsigned)nzh);
+        const int in = r == 0 ? 1 : r == nzh - 1 ? -1 : 0;   // towards the domain
+        // a field's value on this row, written if it is a halo row
+        auto value = [&](double* p, bool odd) {
+            if (in == 0) return p[i];
+            const double v = odd ? -p[i + 2 * in] : 2.0 * p[i + in] - p[i + 2 * in];
+            p[i] = v;
+            return v;
+        };
+        const double dudy = value(A.vg[I_DUDY], false), dwdx = value(A.vg[I_DWDX], true), dwdy = value(A.vg[I_DWDY], true);
+        if (in != 0) {
+            value(A.vg[I_DUDX], false);
+            value(A.vg[I_DVDY], false);
+            value(A.vel[0], false);
+            value(A.vel[1], false);
+            value(A.vel[2], true);
+        }
+        A.vg[I_DUDZ][i] = dwdx + A.vort[1][i];
+        A.vg[I_DVDX][i] = dudy + A.vort[2][i];
+        A.vg[I_DVDZ][i] = dwdy - A.vort[0][i];
     }
 }
 
@@ -1874,14 +1899,10 @@ static void vor2vel_t(Ctx& c) {
                           c.velgrad(I_DWDX), c.velgrad(I_DVDY), c.velgrad(I_DWDY)};
         fft_xy(c, in, out, 8, false);
     }
-    halo(c, {{c.velgrad(I_DUDX), 0}, {c.velgrad(I_DUDY), 0}, {c.velgrad(I_DWDX), 1},
-             {c.velgrad(I_DVDY), 0}, {c.velgrad(I_DWDY), 1},
-             {c.velog(0), 0}, {c.velog(1), 0}, {c.velog(2), 1}});
-    MPtr8 vg;
-    Ptr8 vo;
-    for (int k = 0; k < 8; ++k) vg.p[k] = c.velgrad(k);
-    for (int k = 0; k < 3; ++k) vo.p[k] = c.vortg(k);
-    k_velgrad_fill<<<nblocks(P.fsz), 256, 0, c.stream>>>(vg, vo, P.fsz);
+    VelTail V;
+    for (int k = 0; k < 3; ++k) { V.vel[k] = c.velog(k); V.vort[k] = c.vortg(k); }
+    for (int k = 0; k < 8; ++k) V.vg[k] = c.velgrad(k);
+    k_velgrad_fill<<<nblocks(P.fsz), 256, 0, c.stream>>>(V, P.nzh, P.fsz);
     CKL();
 }
 
