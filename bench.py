@@ -862,9 +862,9 @@ def main():
     ap.add_argument("--spinup", type=int, default=0, help="untimed steps before the warm-up (developed flow)")
     ap.add_argument("--no-autotune", action="store_true", help="keep the default launch shapes")
     ap.add_argument("--scatter-groups", type=int, default=None, choices=range(6),
-                    help="log2 of the consecutive parcels a lane group of the scatters takes (overrides the tuner)")
+                    help="accepted for older command lines; the scatters take 32 consecutive parcels per warp")
     ap.add_argument("--fft-path", type=int, default=None, choices=range(4),
-                    help="horizontal FFT: 0 plane, 1 tiled lines, 2 Stockham lines, 3 half-plane clusters "
+                    help="horizontal FFT: 0 plane, 1 tiled lines, 2 lines of any length, 3 half-plane clusters "
                          "(overrides the tuner)")
     ap.add_argument("--parcels-per-cell", type=int, default=0,
                     help="device-generated initial state with this many parcels per cell (profiling the grid "
