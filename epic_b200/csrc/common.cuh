@@ -134,8 +134,8 @@ EPIC_DEV void set_err(unsigned* err, unsigned bit) { atomicOr(err, bit); }
 
 // Maximum of non-negative doubles through their ordered bits.  A value that does
 // not raise the maximum, nearly every one of a launch's, is dropped by a read of
-// the (possibly older, so smaller) maximum: atomics on one address serialise, and
-// one per warp took 30 us of a step's first bound pass on 900,000 parcels.
+// the (possibly older, so smaller) maximum: atomics on one address serialise (a
+// step's first bound pass on 885,000 parcels: 59 -> 42 us).
 EPIC_DEV void atomic_max_nonneg(unsigned long long* addr, double v) {
     const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
     if (bits > __ldcg(addr)) atomicMax(addr, bits);

@@ -133,8 +133,10 @@ struct Ctx {
     bool pstep_valid = false;
     // Set during the stages of a step: a deformed flow, in which at the step's
     // first par2grid more than a quarter of the parcels had support points in several cells.  Chooses between kernels that
-    // compute the same sums (rounding aside), each the faster one on its side: at
-    // a quarter the stage kernels of a deformed 64^3 flow cost the same.
+    // compute the same sums (rounding aside): the one with gather_shared is 27%
+    // faster on a deformed 64^3 flow and 6% to 10% slower where parcels share
+    // cells.  A quarter of the parcels is gather_shared's own rule (more than 8 of a
+    // warp's 32), which measured alike from 2 to 16.
     bool spread = false;
     bool count_spread = false;    // the next par2grid scatter counts them
     cudaEvent_t spread_ev = nullptr;
